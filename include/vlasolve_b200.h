@@ -120,12 +120,12 @@ int vls_create(const vls_grid_desc *grid, const vls_solver_desc *solver,
      prefilter         VLS_PREFILTER_AUTO: register-resident chunked solves
                        where a line fits them, else shared-memory segments;
                        VLS_PREFILTER_SEGMENT: segments for every line.
-     drift             VLS_DRIFT_AUTO: FP32 storage stages each block's whole
-                       coefficient strip (two blocks per SM where they fit,
-                       else one block of 32 warps), FP64 storage and strips
-                       too tall for one block take staged 64 x 40 windows;
-                       VLS_DRIFT_WINDOW / _STRIP2 / _STRIP1 ask for one of
-                       those (a strip that does not fit falls back to windows).
+     drift             VLS_DRIFT_AUTO: FP32 storage stages whole coefficient
+                       strips (two strip buffers per block where they fit,
+                       else one), FP64 storage and strips too tall for one
+                       block take staged 64 x 40 windows; VLS_DRIFT_WINDOW /
+                       _STRIP2 / _STRIP1 ask for one of those (a strip that
+                       does not fit, or FP64, falls back to windows).
      slices_per_batch  J slices per batch of the prefilter and drift scratch
                        (0: all slices in one batch); the G and C scratch
                        holds streams x slices_per_batch slices.

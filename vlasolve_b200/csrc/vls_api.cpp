@@ -39,11 +39,19 @@ struct vls_handle {
   int32_t *idx = nullptr;        // FP64 footpoints
   void *fx = nullptr, *fy = nullptr;
   uint2 *fp2 = nullptr;          // FP32 packed footpoints
+  // the strip drift's tables for these footpoints: trip kinds, and the
+  // far-tap cells (their number per slice on the host)
+  uint8_t *trip_kinds = nullptr;
+  uint32_t *far_base = nullptr, *far_count = nullptr, *far = nullptr;
+  size_t far_cap = 0;
+  std::vector<uint32_t> far_base_h;
   int64_t nch = 0, nel = 0;
   int64_t *ch_start = nullptr;
   int32_t *ch_len = nullptr;
   void *ch_val = nullptr;
   int32_t *t_idx = nullptr;  // [nch] codes then [nch] slice index
+  uint32_t *ch_at = nullptr;      // each chain's cell within its slice
+  int32_t *d_chain_lo = nullptr;  // chain_lo on the device
   double *t_x = nullptr, *t_y = nullptr;
   double *rp_r = nullptr, *q_r = nullptr, *rp_u = nullptr, *q_u = nullptr;
   double *dU_val = nullptr, *dR_val = nullptr, *dJ_val = nullptr;
@@ -79,10 +87,9 @@ struct vls_handle {
   RcDir<double> rcu_d{}, rcr_d{};
   RcDir<float> rcu_f{}, rcr_f{};
   int rcu_cfg = -1, rcr_cfg = -1;
-  // TMA descriptors of each slot of C for the drift's staged windows (tmC)
-  // and strips (tmS, when drift_kind is a strip kind)
+  // TMA descriptors of each slot of C for the drift's staged windows
   CUtensorMap tmC[8];
-  CUtensorMap tmS[8];
+  CUtensorMap tmS[8];  // and strips (drift_kind a strip kind)
   int drift_kind = DRIFT_WINDOW;
   uint32_t drift_spins = MBAR_SPIN_LIMIT;  // polls of each bounded wait of the drift
   vls_layout_desc layout{};                // what vls_get_layout reports
@@ -299,6 +306,39 @@ static uint2 encode_packed(const Coords &c, int32_t code, double rF, double uF) 
   return w;
 }
 
+// The footpoint tables are new: the strip drift's tables follow them.
+static int footpoints_changed(vls_handle *h) {
+  h->fp_gen++;
+  const Coords &c = h->co;
+  h->far_base_h.assign((size_t)c.nj + 1, 0);
+  if (h->drift_kind == DRIFT_WINDOW) return VLS_OK;
+  if (!h->trip_kinds) {
+    TRY(dalloc(h, &h->trip_kinds, trip_kinds_bytes(c.nr, c.nu, c.nj)));
+    TRY(dalloc(h, &h->far_count, sizeof(uint32_t) * c.nj));
+    TRY(dalloc(h, &h->far_base, sizeof(uint32_t) * (c.nj + 1)));
+  }
+  CK(h, launch_trip_kinds(h->fp2, h->trip_kinds, c.nr, c.nu, c.nj, h->st));
+  CK(h, launch_far_cells(h->fp2, nullptr, h->far_count, nullptr, c.nr, c.nu, c.nj, h->st));
+  CK(h, cudaMemcpyAsync(h->far_base_h.data() + 1, h->far_count, sizeof(uint32_t) * c.nj,
+                        cudaMemcpyDeviceToHost, h->st));
+  CK(h, cudaStreamSynchronize(h->st));
+  size_t total = 0;
+  for (int j = 0; j < c.nj; j++) {
+    total += h->far_base_h[j + 1];
+    if (total > 0xffffffffu) return fail(h, VLS_EINVAL, "too many far footpoints");
+    h->far_base_h[j + 1] = (uint32_t)total;
+  }
+  if (total > h->far_cap || !h->far) {
+    // grown for footpoints with more such cells (an outgrown list is freed
+    // with the handle)
+    h->far_cap = total;
+    TRY(dalloc(h, &h->far, sizeof(uint32_t) * std::max<size_t>(total, 1)));
+  }
+  TRY(upload(h, h->far_base, h->far_base_h.data(), sizeof(uint32_t) * (c.nj + 1)));
+  CK(h, launch_far_cells(h->fp2, h->far_base, nullptr, h->far, c.nr, c.nu, c.nj, h->st));
+  return VLS_OK;
+}
+
 // Encoding of one cell: -1 -> outside the box (value 0), <= -2 -> delayed
 // kernel chain (-2 - chain id), else rI | uI << 16 (FP64 tables); the FP32
 // tables pack the same information into two 32-bit words.
@@ -384,8 +424,7 @@ static int encode_and_upload_footpoints(vls_handle *h, bool build_chains) {
       TRY(upload(h, h->fp2 + off, packed.data(), n * sizeof(uint2)));
     }
   }
-  h->fp_gen++;
-  return VLS_OK;
+  return footpoints_changed(h);
 }
 
 // localSpline::evaluate(R, U) position decomposition of every chain tail
@@ -434,12 +473,22 @@ static int setup_chain_device(vls_handle *h) {
   TRY(dalloc(h, &h->ch_len, sizeof(int32_t) * std::max<int64_t>(nch, 1)));
   TRY(dalloc(h, &h->ch_val, es * std::max<int64_t>(h->nel, 1)));
   TRY(dalloc(h, &h->t_idx, sizeof(int32_t) * tcode.size()));
+  TRY(dalloc(h, &h->ch_at, sizeof(uint32_t) * std::max<int64_t>(nch, 1)));
+  TRY(dalloc(h, &h->d_chain_lo, sizeof(int32_t) * (c.nj + 1)));
   TRY(dalloc(h, &h->t_x, sizeof(double) * tx.size()));
   TRY(dalloc(h, &h->t_y, sizeof(double) * ty.size()));
   CK(h, cudaMemsetAsync(h->ch_val, 0, es * std::max<int64_t>(h->nel, 1), h->st));
   if (nch) {
     TRY(upload(h, h->ch_start, h->ch_start_h.data(), sizeof(int64_t) * nch));
     TRY(upload(h, h->ch_len, h->ch_len_h.data(), sizeof(int32_t) * nch));
+    std::vector<uint32_t> at((size_t)nch);
+    for (int64_t k = 0; k < nch; k++)
+      at[k] = (uint32_t)(h->ch_cell_h[k] % ((int64_t)c.nr * c.nu));
+    TRY(upload(h, h->ch_at, at.data(), sizeof(uint32_t) * nch));
+  }
+  {
+    const std::vector<int32_t> lo(h->chain_lo.begin(), h->chain_lo.end());
+    TRY(upload(h, h->d_chain_lo, lo.data(), sizeof(int32_t) * lo.size()));
   }
   TRY(upload(h, h->t_idx, tcode.data(), sizeof(int32_t) * tcode.size()));
   TRY(upload(h, h->t_x, tx.data(), sizeof(double) * tx.size()));
@@ -448,8 +497,8 @@ static int setup_chain_device(vls_handle *h) {
 }
 
 // 3D tiled tensor maps of C ([N_J][N_u+3][pc], element T): boxes of 64
-// columns x 40 rows x 1 slice for the drift windows, 48 columns x 64 rows x 1
-// slice for the strips.  The encoder is the driver's cuTensorMapEncodeTiled,
+// columns x 40 rows x 1 slice for the drift windows, 48 columns x
+// drift_strip_box_rows x 1 slice for the strips.  The encoder is the driver's cuTensorMapEncodeTiled,
 // reached through the runtime (no libcuda link).  Returns false when it is
 // unavailable or refuses a map (vls_create then fails: every drift kernel
 // stages its coefficients by TMA).
@@ -481,12 +530,11 @@ static bool make_tensor_map(vls_handle *h) {
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return false;
     if (h->drift_kind != DRIFT_WINDOW) {
-      const cuuint32_t sbox[3] = {48, 64, 1};
-      if (enc(&h->tmS[s],
-              es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
-              base, dims, strides, sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      const cuuint32_t sbox[3] = {48, (cuuint32_t)drift_strip_box_rows(h->co.nu), 1};
+      if (enc(&h->tmS[s], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, sbox, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
+          CUDA_SUCCESS)
         return false;
     }
   }
@@ -675,7 +723,7 @@ extern "C" int vls_create_layout(const vls_grid_desc *grid, const vls_solver_des
   A(dalloc(hp, &h->d_dU, sizeof(double) * c.nu));
   A(dalloc(hp, &h->d_Ct1, sizeof(double) * c.nj));
   A(dalloc(hp, &h->bu, sizeof(double) * c.nu));
-  A(dalloc(hp, &h->bu32, sizeof(float) * c.nu));
+  A(dalloc(hp, &h->bu32, sizeof(float) * ((c.nu + 7) / 8 * 8)));  // whole trips of 8 rows
   A(dalloc(hp, &h->wj, sizeof(double) * c.nj));
   A(dalloc(hp, &h->dR4, sizeof(double) * c.nr));
   A(dalloc(hp, &h->Rcoef, sizeof(double) * c.nr));
@@ -758,8 +806,9 @@ extern "C" int vls_create_layout(const vls_grid_desc *grid, const vls_solver_des
   U2(h->d_Ct1, Ct1.data(), sizeof(double) * c.nj);
   U2(h->bu, bu.data(), sizeof(double) * c.nu);
   {
-    const std::vector<float> b32(bu.begin(), bu.end());
-    U2(h->bu32, b32.data(), sizeof(float) * c.nu);
+    std::vector<float> b32(bu.begin(), bu.end());
+    b32.resize((size_t)(c.nu + 7) / 8 * 8, 0.f);
+    U2(h->bu32, b32.data(), sizeof(float) * b32.size());
   }
   U2(h->wj, wj.data(), sizeof(double) * c.nj);
   U2(h->dR4, dR4.data(), sizeof(double) * c.nr);
@@ -1062,8 +1111,7 @@ extern "C" int vls_set_footpoints(vls_handle *h, const int32_t *rI,
     for (size_t i = 0; i < h->cells; i++) p[i] = encode_packed(c, idx[i], rF[i], uF[i]);
     TRY(upload(h, h->fp2, p.data(), sizeof(uint2) * h->cells));
   }
-  h->fp_gen++;
-  return VLS_OK;
+  return footpoints_changed(h);
 }
 
 // ------------------------------------------------------------------ step
@@ -1120,32 +1168,34 @@ static int drift_once(vls_handle *h, bool kick, const void *f_in = nullptr,
                 return launch_prer<T, R>(G, C, g, tr, bs);
               },
               bs));
-    const int64_t c_lo = h->chain_lo[g.j0], c_hi = h->chain_lo[g.j0 + g.nb];
-    if (c_hi > c_lo) {
+    int64_t most = 0;
+    for (int j = g.j0; j < g.j0 + g.nb; j++)
+      most = std::max<int64_t>(most, h->chain_lo[j + 1] - h->chain_lo[j] +
+                                         (int64_t)(h->far_base_h[j + 1] - h->far_base_h[j]));
+    if (most > 0) {
+      const EdgeTables et{h->ch_start, h->ch_len,      h->ch_at,    h->t_idx, h->t_x,
+                          h->t_y,      h->d_chain_lo, h->far_base, h->far};
       CK(h, timed(
                 h, VLS_K_TAILS,
                 [&] {
-                  return launch_chain_tails<T>(C, (T *)h->ch_val, h->ch_start, h->ch_len,
-                                               h->t_idx, h->t_x, h->t_y, h->nch, c_lo,
-                                               c_hi, h->ndrift, g, bs);
+                  return launch_edge<T>(C, fout, (T *)h->ch_val, et, h->ndrift, h->fp2,
+                                        (int)most, g, bs);
                 },
                 bs));
     }
     CK(h, timed(
               h, VLS_K_DRIFT,
               [&] {
-                if (h->drift_kind != DRIFT_WINDOW)
-                  return launch_drift_strip<T>(&h->tmS[sl], h->drift_kind, C, fout,
-                                               h->idx, (const T *)h->fx, (const T *)h->fy,
-                                               h->fp2, h->ch_start, h->ch_len,
-                                               (const T *)h->ch_val, h->ndrift,
-                                               moment_tables(h), h->partial, h->flag + 1,
-                                               h->drift_spins, g, bs);
-                return launch_drift_tma<T>(&h->tmC[sl], C, fout, h->idx,
-                                           (const T *)h->fx, (const T *)h->fy, h->fp2,
-                                           h->ch_start, h->ch_len, (const T *)h->ch_val,
-                                           h->ndrift, moment_tables(h), h->partial,
-                                           h->flag + 1, h->drift_spins, g, bs);
+                if constexpr (sizeof(T) == 4) {
+                  if (h->drift_kind != DRIFT_WINDOW)
+                    return launch_drift_strip(&h->tmS[sl], h->drift_kind, C, fout, h->fp2,
+                                              h->trip_kinds, moment_tables(h), h->partial,
+                                              h->flag + 1, h->drift_spins, g, bs);
+                }
+                return launch_drift_tma<T>(&h->tmC[sl], C, fout, h->idx, (const T *)h->fx,
+                                           (const T *)h->fy, h->fp2, h->ch_start, h->ch_len,
+                                           (const T *)h->ch_val, h->ndrift, moment_tables(h),
+                                           h->partial, h->flag + 1, h->drift_spins, g, bs);
               },
               bs));
   }

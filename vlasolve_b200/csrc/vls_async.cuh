@@ -27,6 +27,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
                "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -45,6 +48,20 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     if (i >= 32) __nanosleep(20);
   }
   return false;
+}
+// the same for warps that wait for microseconds next to working ones, whose
+// issue slots closer polls would take
+__device__ __forceinline__ bool mbar_wait_idle(uint64_t *bar, uint32_t parity,
+                                               uint32_t limit = MBAR_SPIN_LIMIT) {
+  for (uint32_t i = 0; i < limit; ++i) {
+    if (mbar_test_wait(bar, parity)) return true;
+    __nanosleep(100);
+  }
+  return false;
+}
+// brings [src, src + bytes) into L2 (both multiples of 16)
+__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -108,26 +108,44 @@ cudaError_t launch_drift_tma(const CUtensorMap *tmC, const T *C, T *f, const int
                              const T *ch_val, int64_t ndrift, const MomentTables &mt,
                              double *partial, unsigned int *err, uint32_t spins,
                              const Geometry &g, cudaStream_t st);
-// drift with the block's whole coefficient strip staged by TMA (tmS: 3D map
-// of C with box 48 columns x 64 rows x 1 slice).  drift_strip_width returns
-// the strip kind (DRIFT_STRIP2 / DRIFT_STRIP1) the grid takes, or
-// DRIFT_WINDOW when none fits; want != DRIFT_AUTO requests one kind
+// drift from whole coefficient strips staged by TMA (tmS: 3D map of C, box 48
+// columns x drift_strip_box_rows x 1 slice).  drift_strip_width returns the
+// strip kind (DRIFT_STRIP2 / DRIFT_STRIP1) the grid takes, or DRIFT_WINDOW
+// when none fits; want != DRIFT_AUTO requests one kind
 template <typename T>
 int drift_strip_width(int nu, int want);
+int drift_strip_box_rows(int nu);
+cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C, float *f,
+                               const uint2 *fp2, const uint8_t *trip_kinds,
+                               const MomentTables &mt, double *partial, unsigned int *err,
+                               uint32_t spins, const Geometry &g, cudaStream_t st);
+// what the strip drift knows of its footpoints (see vls_kernels.cu), from the
+// packed tables of all slices: the kind of each trip (bytes of that table,
+// and the kernel that fills it), and the cells of each slice whose taps leave
+// their strip (their number per slice, or with a list and its base per slice
+// the entries)
+size_t trip_kinds_bytes(int nr, int nu, int nj);
+cudaError_t launch_trip_kinds(const uint2 *fp2, uint8_t *kinds, int nr, int nu, int nj,
+                              cudaStream_t st);
+cudaError_t launch_far_cells(const uint2 *fp2, const uint32_t *base, uint32_t *count,
+                             uint32_t *list, int nr, int nu, int nj, cudaStream_t st);
+// the chains (their ring, cell within the slice, tail footpoint; chain_lo:
+// first chain of each slice) and, for the strip drift, the far-tap cells
+// (far_base: first of each slice; nullptr for the windowed drift).
+// launch_edge advances every chain of the launch's slices and, for the strip
+// drift, writes the edge cells' values into f (edge_kernel)
+struct EdgeTables {
+  const int64_t *ch_start;
+  const int32_t *ch_len;
+  const uint32_t *ch_at;
+  const int32_t *t_idx;
+  const double *t_x, *t_y;
+  const int32_t *chain_lo;
+  const uint32_t *far_base, *far;
+};
 template <typename T>
-cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const T *C, T *f,
-                               const int32_t *idx, const T *fx, const T *fy, const uint2 *fp2,
-                               const int64_t *ch_start, const int32_t *ch_len,
-                               const T *ch_val, int64_t ndrift, const MomentTables &mt,
-                               double *partial, unsigned int *err, uint32_t spins,
-                               const Geometry &g, cudaStream_t st);
-// chains [c_lo, c_hi) (all of the launch's slices) of nchains in total
-template <typename T>
-cudaError_t launch_chain_tails(const T *C, T *ch_val, const int64_t *ch_start,
-                               const int32_t *ch_len, const int32_t *t_idx,
-                               const double *t_x, const double *t_y,
-                               int64_t nchains, int64_t c_lo, int64_t c_hi,
-                               int64_t ndrift, const Geometry &g, cudaStream_t st);
+cudaError_t launch_edge(const T *C, T *f, T *ch_val, const EdgeTables &t, int64_t ndrift,
+                        const uint2 *fp2, int most, const Geometry &g, cudaStream_t st);
 struct HostDirTables;
 // chunk layout of the register kernels for a direction (-1: none takes it,
 // the shared-memory segment kernels then solve the lines; u_lines for the

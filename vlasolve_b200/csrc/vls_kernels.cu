@@ -20,6 +20,7 @@
 // K = 32 rows reach FP64 rounding and K = 20 rows reach 1e-11).  The per-row
 // coefficients are the reference's own (tabulated on the host in its
 // operation order).  Recursions run in FP64 in both precisions.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 
@@ -574,14 +575,21 @@ constexpr int DR_W = 8;  // warps per drift block
 
 // FP32 tables, 8 bytes per cell: word = index << FP_FBITS | round(frac * 2^FP_FBITS)
 // per direction; FP_OUT / FP_CHAIN in the first word mark the two special kinds
-// (the second word then holds the chain id).  The 21 fraction bits are placed
-// straight into a float mantissa (value 1.frac, minus 1): no int->float convert.
+// (the second word then holds the chain id).  The 21 fraction bits are the low
+// mantissa bits of a float in [4, 5), whose spacing is 2^-21: one logic
+// operation and a subtraction of 4, no shift and no int->float convert.
 constexpr int FP_FBITS = 21;
 constexpr uint32_t FP_FMASK = (1u << FP_FBITS) - 1u;
 constexpr uint32_t FP_OUT = 0xFFFFFFFFu, FP_CHAIN = 0xFFFFFFFEu;
 
 __device__ __forceinline__ float frac21(uint32_t w) {
-  return __uint_as_float(0x3F800000u | ((w & FP_FMASK) << 2)) - 1.0f;
+  return __uint_as_float(0x40800000u | (w & FP_FMASK)) - 4.0f;
+}
+// both directions' fractions of one cell
+__device__ __forceinline__ float2 frac21x2(uint2 w) {
+  return __fadd2_rn(make_float2(__uint_as_float(0x40800000u | (w.x & FP_FMASK)),
+                                __uint_as_float(0x40800000u | (w.y & FP_FMASK))),
+                    make_float2(-4.f, -4.f));
 }
 
 // ------------------------------------------------------- TMA-staged drift
@@ -680,12 +688,13 @@ __device__ __forceinline__ float eval_window<float>(const float *p, float x, flo
 template <typename T>
 __global__ void __launch_bounds__(DT_THREADS)
     drift_tma_kernel(const __grid_constant__ CUtensorMap tmC, const T *__restrict__ C,
-                     T *__restrict__ f, const int32_t *__restrict__ idx,
-                     const T *__restrict__ fx, const T *__restrict__ fy,
-                     const uint2 *__restrict__ fp2, const int64_t *__restrict__ ch_start,
-                     const int32_t *__restrict__ ch_len, const T *__restrict__ ch_val,
-                     int64_t ndrift, MomentTables mt, double *__restrict__ partial,
-                     unsigned int *err, uint32_t spins, Geometry g) {
+                     T *__restrict__ f,
+                     const int32_t *__restrict__ idx, const T *__restrict__ fx,
+                     const T *__restrict__ fy, const uint2 *__restrict__ fp2,
+                     const int64_t *__restrict__ ch_start, const int32_t *__restrict__ ch_len,
+                     const T *__restrict__ ch_val, int64_t ndrift, MomentTables mt,
+                     double *__restrict__ partial, unsigned int *err, uint32_t spins,
+                     Geometry g) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   T *win = reinterpret_cast<T *>(smem_raw);  // two windows
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + 2 * DW_COLS * DW_ROWS * sizeof(T));
@@ -811,434 +820,651 @@ cudaError_t launch_drift_tma(const CUtensorMap *tmC, const T *C, T *f, const int
 }
 
 // ------------------------------------------------------------ strip drift
-// Block: 32 output columns x every row of one J slice.  The block's whole
-// coefficient strip (WC columns starting (WC-32)/2 columns to the left, all
-// N_u+3 rows) is staged once by TMA in DS_ROWS-row boxes, one mbarrier per
-// box, so a cell can read any row of the strip: the footpoints' u
-// displacements reach hundreds of rows while their r displacements stay
-// within a few columns.  A cell waits only for the boxes its taps lie in
-// (bounded; after a timeout the thread reads C in global memory).  No block
-// barrier is taken inside the row loop.  Cells whose taps leave the strip's
-// columns gather from global memory.
-constexpr int DS_ROWS = 64;
-
-template <typename T, int PITCH>
-__device__ __forceinline__ T eval_pitch(const T *p, T x, T y) {
-  const T b2xI = bv2<T>(T(1) - x), b1xI = bv1<T>(T(1) - x);
-  const T b1x = bv1<T>(x), b2x = bv2<T>(x);
-  const T s0 = p[0] * b2xI + p[1] * b1xI + p[2] * b1x + p[3] * b2x;
-  const T s1 = p[PITCH] * b2xI + p[PITCH + 1] * b1xI + p[PITCH + 2] * b1x + p[PITCH + 3] * b2x;
-  const T s2 = p[2 * PITCH] * b2xI + p[2 * PITCH + 1] * b1xI + p[2 * PITCH + 2] * b1x +
-               p[2 * PITCH + 3] * b2x;
-  const T s3 = p[3 * PITCH] * b2xI + p[3 * PITCH + 1] * b1xI + p[3 * PITCH + 2] * b1x +
-               p[3 * PITCH + 3] * b2x;
-  return over36<T>(bv2<T>(T(1) - y) * s0 + bv1<T>(T(1) - y) * s1 +
-                           bv1<T>(y) * s2 + bv2<T>(y) * s3);
-}
+// FP32 storage: the coefficient strip of 32 output columns (DS_WC columns
+// starting DS_XL to the left, all N_u + 3 rows) is staged in shared memory, so
+// that a cell can read any row of it: the footpoints' u displacements
+// reach hundreds of rows while their r displacements stay within a few
+// columns.  Cells whose taps leave the strip's columns gather from global
+// memory.
 template <int PITCH>
 __device__ __forceinline__ float eval_pitch_f32x2(const float *p, float x, float y) {
   return gather_f32x2([&](int a, int b) { return p[a * PITCH + b]; }, x, y);
 }
-template <typename T, int PITCH>
-__device__ __forceinline__ T eval_strip(const T *p, T x, T y) {
-  if constexpr (sizeof(T) == 4)
-    return eval_pitch_f32x2<PITCH>(p, x, y);
-  else
-    return eval_pitch<T, PITCH>(p, x, y);
-}
 
-// Footpoint fields needed by the strip's fast path: the gather test and the
-// tap position.  For non-gather words the values are unused.
-template <typename T>
-struct FastFoot {
-  bool gather;
-  int rI, uI;
-  T x, y;
-};
-__device__ __forceinline__ FastFoot<float> fast_foot(const RawCell<float> &c) {
-  FastFoot<float> p;
-  p.gather = c.w.x < FP_CHAIN;
-  p.rI = (int)(c.w.x >> FP_FBITS);
-  p.uI = (int)(c.w.y >> FP_FBITS);
-  // both fractions with one packed subtraction of 1 (values 1.frac21)
-  const float2 xy = __fadd2_rn(
-      make_float2(__uint_as_float(0x3F800000u | ((c.w.x & FP_FMASK) << 2)),
-                  __uint_as_float(0x3F800000u | ((c.w.y & FP_FMASK) << 2))),
-      make_float2(-1.f, -1.f));
-  p.x = xy.x;
-  p.y = xy.y;
-  return p;
+// The kinds of a trip, DS_TRIP rows of one strip (32 columns) of a slice:
+// nothing to compute (every cell outside the box: 0), regular (every cell
+// gathers inside the strip, and from row to row each column's 4 x 4 taps move
+// by exactly one coefficient row), anything else.  Footpoints vary so slowly
+// along u that 57 % of the trips are regular and 18 % empty on the
+// 513 x 513 x 256 Hernquist grid (48 % and 17 % on 257 x 257 x 128 Plummer).
+// They are fixed for the run, so the kinds are found once per table.
+constexpr int DS_TRIP = 8;
+enum { TRIP_ANY = 0, TRIP_REGULAR = 1, TRIP_EMPTY = 2 };
+__host__ __device__ inline int strip_blocks(int nr) {
+  // N_r = 32 k + 1 (every grid of the form 2^n + 1): k strips, the last one's
+  // block also takes the last column; 2.4 % faster than a block of one column
+  // on the 513 x 513 x 256 case
+  return (nr % 32 == 1 && nr > 32) ? nr / 32 : (nr + 31) / 32;
 }
-__device__ __forceinline__ FastFoot<double> fast_foot(const RawCell<double> &c) {
-  FastFoot<double> p;
-  p.gather = c.code >= 0;
-  p.rI = c.code & 0xffff;
-  p.uI = c.code >> 16;
-  p.x = c.x;
-  p.y = c.y;
-  return p;
-}
+__host__ __device__ inline int strip_trips(int nu) { return (nu + DS_TRIP - 1) / DS_TRIP; }
+constexpr int DS_WC = 48, DS_XL = (DS_WC - 32) / 2;  // columns staged, and left of the strip
+// consumer warps of a block (one producer warp besides) and footpoint rows in
+// flight per warp: drift of 513 x 513 x 256 Hernquist / 257 x 257 x 128
+// Plummer with 31 warps and two rows (64 registers) 0.295 / 0.061 ms, 23 and
+// four (80 registers) 0.270 / 0.053, 19 and four (96) 0.261 / 0.049, 17 and
+// four 0.277 / 0.051, 13 and four 0.309 / 0.052, 19 and eight 0.282 / 0.051
+constexpr int STRIP_WARPS = 19;
+constexpr int DS_AHEAD = 4;
 
-// The in-strip gather of one cell, run for every lane with the tap offset
-// zeroed where it does not apply; `slow`: the cell takes strip_slow instead
-// (outside, chain front, taps outside the strip's columns, or every cell
-// after a failed wait: wcap = 0).
-template <typename T, int WC>
-__device__ __forceinline__ T strip_fast(const RawCell<T> &c, const T *win, int x0,
-                                        uint32_t wcap, bool col_ok, bool &slow) {
-  const FastFoot<T> p = fast_foot(c);
-  const int wc = p.rI - x0;
-  const bool in = col_ok && p.gather && (uint32_t)wc < wcap;
-  const int so = in ? p.uI * WC + wc : 0;
-  slow = col_ok && !in;
-  return eval_strip<T, WC>(win + so, p.x, p.y);
-}
-
-// A cell the in-strip gather does not cover: the gather from C in global
-// memory, a chain front, or zero outside.
-template <typename T>
-__device__ __forceinline__ T strip_slow(const RawCell<T> &c, const T *__restrict__ Cj,
-                                        const int64_t *__restrict__ ch_start,
-                                        const int32_t *__restrict__ ch_len,
-                                        const T *__restrict__ ch_val, int64_t ndrift,
-                                        const Geometry &g) {
-  const Cell<T> cl = decode(c);
-  T v = T(0);
-  if (cl.kind == 0)
-    v = eval2d<T>(Cj, g.pc, cl.rI, cl.x, cl.uI, cl.y);
-  else if (cl.kind == 2)
-    v = ch_val[__ldg(ch_start + cl.ch) + ndrift % __ldg(ch_len + cl.ch)];
-  return v;
-}
-
-// One cell of the strip drift once every box has landed (wcap = WC - 3, or 0
-// after a failed wait, which sends every cell to the global-memory gather).
-// A warp vote sends the rare cells the in-strip gather does not cover through
-// the general decode.  Every lane of the warp must call it.
-template <typename T, int WC>
-__device__ __forceinline__ T strip_cell(const RawCell<T> &c, const T *win, int x0,
-                                        uint32_t wcap, bool col_ok, const T *__restrict__ Cj,
-                                        const int64_t *__restrict__ ch_start,
-                                        const int32_t *__restrict__ ch_len,
-                                        const T *__restrict__ ch_val, int64_t ndrift,
-                                        const Geometry &g) {
-  bool slow;
-  T v = strip_fast<T, WC>(c, win, x0, wcap, col_ok, slow);
-  if (__any_sync(0xffffffffu, slow))
-    if (slow) v = strip_slow<T>(c, Cj, ch_start, ch_len, ch_val, ndrift, g);
-  return v;
-}
-
-// b_u in the storage type (a copy rounded once on the host for FP32)
-template <typename T>
-__device__ __forceinline__ T moment_bu(const MomentTables &mt, int u) {
-  if constexpr (sizeof(T) == 4)
-    return __ldg(mt.bu32 + u);
-  else
-    return __ldg(mt.bu + u);
-}
-
-// The rows of one strip column (lane) for warp w: rows w, w + NW, ...,
-// footpoints PF rows ahead in flight.  Offsets are relative to slice j and
-// 32-bit; the prefetch runs past the slice's last row into the next slice
-// or the tables' padding (FOOT_PAD_ROWS rows and 32 cells), and lanes past
-// N_r read the next row's words, which they do not use.
-template <typename T, int WC, int NW, int PF>
-__device__ __forceinline__ void strip_rows(
-    const T *win, int x0, bool waits_ok, bool col_ok, int j, int r, int w,
-    const T *__restrict__ Cj, T *__restrict__ f,
-    const int32_t *__restrict__ idx, const T *__restrict__ fx, const T *__restrict__ fy,
-    const uint2 *__restrict__ fp2, const int64_t *__restrict__ ch_start,
-    const int32_t *__restrict__ ch_len, const T *__restrict__ ch_val, int64_t ndrift,
-    const MomentTables &mt, const Geometry &g, double &acc) {
-  static_assert(NW * PF + 1 <= FOOT_PAD_ROWS, "prefetch reaches past the padding rows");
-  const size_t sb = (size_t)j * g.nu * g.nr;
-  const int32_t *ids = idx;
-  const T *fxs = fx, *fys = fy;
-  const uint2 *fps = fp2;
-  if constexpr (sizeof(T) == 4)
-    fps += sb;
-  else {
-    ids += sb;
-    fxs += sb;
-    fys += sb;
+// one warp per trip (lanes past N_r take the last column, as the drift does)
+__global__ void __launch_bounds__(256)
+    trip_kind_kernel(const uint2 *__restrict__ fp2, uint8_t *__restrict__ kinds, int nr, int nu,
+                     int nj) {
+  const int ns = strip_blocks(nr), nt = strip_trips(nu);
+  const size_t k = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (k >= (size_t)nj * ns * nt) return;
+  const int t = (int)(k % nt), s = (int)(k / nt % ns);
+  const size_t j = k / ((size_t)nt * ns);
+  const int r = min(32 * s + (int)(threadIdx.x & 31), nr - 1), x0 = 32 * s - DS_XL;
+  bool regular = DS_TRIP * (t + 1) <= nu, empty = true;
+  uint32_t px = 0, py = 0;
+  for (int q = 0; q < DS_TRIP && DS_TRIP * t + q < nu; ++q) {
+    const uint2 w = __ldg(fp2 + (j * nu + DS_TRIP * t + q) * nr + r);
+    const uint32_t ix = w.x >> FP_FBITS, iy = w.y >> FP_FBITS;
+    empty = empty && w.x == FP_OUT;
+    regular = regular && w.x < FP_CHAIN && ix - (uint32_t)x0 < (uint32_t)(DS_WC - 3) &&
+              (q == 0 || (ix == px && iy == py + 1u));
+    px = ix;
+    py = iy;
   }
-  T *fs = f + sb;
-  const uint32_t step = (uint32_t)NW * (uint32_t)g.nr;
-  const uint32_t ahead = (uint32_t)PF * step;
-  const uint32_t wcap = waits_ok ? (uint32_t)(WC - 3) : 0u;
-  uint32_t off = (uint32_t)w * (uint32_t)g.nr + (uint32_t)r;
-  RawCell<T> q[PF];
-#pragma unroll
-  for (int k = 0; k < PF; ++k) q[k] = load_raw(ids, fxs, fys, fps, off + k * step);
-  int u = w;
-  // groups whose PF rows all lie in the slice: the PF in-strip gathers, one
-  // warp vote for the group's rare cells, then the stores (an L2 prefetch of
-  // the footpoint words further ahead measured 4 % slower)
-  for (; u + NW * (PF - 1) < g.nu; u += NW * PF) {
-    T v[PF];
-    bool slow[PF];
-    RawCell<T> c[PF];
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < PF; ++k) {
-      c[k] = q[k];
-      q[k] = load_raw(ids, fxs, fys, fps, off + ahead + k * step);
-      v[k] = strip_fast<T, WC>(c[k], win, x0, wcap, col_ok, slow[k]);
-      any |= slow[k];
-    }
-    if (__any_sync(0xffffffffu, any)) {
-#pragma unroll
-      for (int k = 0; k < PF; ++k)
-        if (slow[k]) v[k] = strip_slow<T>(c[k], Cj, ch_start, ch_len, ch_val, ndrift, g);
-    }
-    T part = T(0);
-#pragma unroll
-    for (int k = 0; k < PF; ++k) {
-      if (col_ok) {
-        fs[off] = v[k];
-        part += moment_bu<T>(mt, u + NW * k) * v[k];
-      }
-      off += step;
-    }
-    acc += (double)part;
-  }
-  // the last, partial group (u is warp-uniform, so the vote in strip_cell
-  // sees the whole warp)
-  T part = T(0);
-#pragma unroll
-  for (int k = 0; k < PF; ++k) {
-    if (u + NW * k < g.nu) {
-      const T v = strip_cell<T, WC>(q[k], win, x0, wcap, col_ok, Cj, ch_start, ch_len, ch_val,
-                                    ndrift, g);
-      if (col_ok) {
-        fs[off] = v;
-        part += moment_bu<T>(mt, u + NW * k) * v;
-      }
-      off += step;
-    }
-  }
-  acc += (double)part;
+  const bool all_regular = __all_sync(0xffffffffu, regular);
+  const bool all_empty = __all_sync(0xffffffffu, empty);
+  if ((threadIdx.x & 31) == 0)
+    kinds[k] = all_regular ? TRIP_REGULAR : all_empty ? TRIP_EMPTY : TRIP_ANY;
 }
 
-template <typename T, int WC, int NW, int MINB, int PF = 2>
-__global__ void __launch_bounds__(32 * NW, MINB)
-    drift_strip_kernel(const __grid_constant__ CUtensorMap tmS, const T *__restrict__ C,
-                       T *__restrict__ f, const int32_t *__restrict__ idx,
-                       const T *__restrict__ fx, const T *__restrict__ fy,
-                       const uint2 *__restrict__ fp2, const int64_t *__restrict__ ch_start,
-                       const int32_t *__restrict__ ch_len, const T *__restrict__ ch_val,
-                       int64_t ndrift, MomentTables mt, double *__restrict__ partial,
-                       unsigned int *err, uint32_t spins, int extra, Geometry g) {
-  constexpr int XL = (WC - 32) / 2;
-  // PF: rows of footpoints in flight per thread.  16 warps with PF = 2 (two
-  // blocks per SM) measured fastest on the 513 x 513 x 256 case: drift 0.309
-  // ms against 0.318 / 0.361 (PF 3 / 1), 0.319 / 0.327 (12 warps, PF 2 / 3),
-  // 0.398 / 0.316 (8 warps, PF 2 / 4)
-  constexpr uint32_t BYTES = DS_ROWS * WC * sizeof(T);
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  __shared__ double red[NW][32];
-  const int rows = g.nu + 3;
-  const int nch = (rows + DS_ROWS - 1) / DS_ROWS;
-  T *win = reinterpret_cast<T *>(smem_raw);
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + (size_t)nch * BYTES);
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int r0 = blockIdx.x * 32, r = r0 + lane;
-  const int jl = blockIdx.y, j = g.j0 + jl;
-  const int x0 = r0 - XL;
-  if (tid == 0) {
-    for (int c = 0; c < nch; ++c) mbar_init(&bar[c], 1);
-    mbar_fence_init();
-    for (int c = 0; c < nch; ++c) {
-      mbar_expect_tx(&bar[c], BYTES);
-      tma_load_3d(win + (size_t)c * DS_ROWS * WC, &tmS, x0, c * DS_ROWS, jl, &bar[c]);
+size_t trip_kinds_bytes(int nr, int nu, int nj) {
+  return (size_t)nj * strip_blocks(nr) * strip_trips(nu);
+}
+
+// Edge cells: those whose value the drift kernels do not gather themselves.
+// Chain fronts, and, with a strip layout, cells whose taps leave the strip's
+// columns (0.4 % of the cells of the 513 x 513 x 256 Hernquist grid, all in
+// its first columns).  edge_kernel writes their values into f before the
+// drift, which reads them there for its moment sums.  Word of such a cell:
+// neither outside nor gathering in the strip.
+__device__ __forceinline__ bool in_strip(uint2 w, int x0) {
+  return w.x < FP_CHAIN && (w.x >> FP_FBITS) - (uint32_t)x0 < (uint32_t)(DS_WC - 3);
+}
+// the far-tap cells of each slice (cell index within the slice): one block
+// per slice; counts them, or fills the slice's part of the list
+__global__ void __launch_bounds__(1024)
+    far_cells_kernel(const uint2 *__restrict__ fp2, const uint32_t *__restrict__ base,
+                     uint32_t *__restrict__ count, uint32_t *__restrict__ list, int nr, int nu) {
+  __shared__ uint32_t n;
+  const int ns = strip_blocks(nr);
+  const uint32_t cells = (uint32_t)nr * (uint32_t)nu;
+  if (threadIdx.x == 0) n = 0u;
+  __syncthreads();
+  const uint2 *ws = fp2 + (size_t)blockIdx.x * cells;
+  for (uint32_t i = threadIdx.x; i < cells; i += blockDim.x) {
+    const uint2 w = __ldg(ws + i);
+    const int x0 = 32 * min((int)(i % (uint32_t)nr) / 32, ns - 1) - DS_XL;
+    if (w.x < FP_CHAIN && !in_strip(w, x0)) {
+      const uint32_t at = atomicAdd(&n, 1u);
+      if (list) list[base[blockIdx.x] + at] = i;
     }
   }
   __syncthreads();
-  const T *Cj = C + (size_t)jl * rows * g.pc;
-  const bool col_ok = r < g.nr;
-  int ready = 0;  // boxes [0, ready) seen complete by this thread
-  bool waits_ok = true;
-  // every box before the first cell (the other block on the SM computes
-  // meanwhile); `spins` bounds each wait
-  for (; ready < nch; ++ready)
-    if (!mbar_wait_bounded(&bar[ready], 0u, spins)) {
-      waits_ok = false;
-      atomicOr(err, 1u);
-      break;
-    }
-  double acc = 0.0;
-  strip_rows<T, WC, NW, PF>(win, x0, waits_ok, col_ok, j, r, w, Cj, f, idx, fx, fy, fp2,
-                            ch_start, ch_len, ch_val, ndrift, mt, g, acc);
-  // extra: the grid has N_r / 32 blocks and N_r = 32 k + 1; the last block
-  // also computes the last column from its strip (columns r0 - 8 .. r0 + 39
-  // cover it), one row per thread, instead of a block of one column
-  double acc2 = 0.0;
-  const bool xblock = extra && blockIdx.x == gridDim.x - 1;
-  if (xblock) {
-    const int rx = r0 + 32;
-    for (int u = tid; u < g.nu; u += 32 * NW) {
-      const size_t cell = ((size_t)j * g.nu + u) * g.nr + rx;
-      const Cell<T> cl = decode(load_raw(idx, fx, fy, fp2, cell));
-      T v = T(0);
-      if (cl.kind == 0) {
-        const int wc = cl.rI - x0;
-        bool inwin = waits_ok && wc >= 0 && wc <= WC - 4;
-        if (inwin) {
-          // every box was awaited above (ready == nch), so these bounded
-          // waits never run; without the loop the compiler's register
-          // allocation of this kernel spills (40 B a thread, the drift 8 %
-          // slower on the 513 x 513 x 256 case)
-          const int cb = (cl.uI + 3) / DS_ROWS;
-          while (ready <= cb) {
-            if (!mbar_wait_bounded(&bar[ready], 0u)) {
-              waits_ok = false;
-              inwin = false;
-              atomicOr(err, 1u);
-              break;
-            }
-            ++ready;
-          }
-        }
-        v = inwin ? eval_strip<T, WC>(win + (size_t)cl.uI * WC + wc, cl.x, cl.y)
-                  : eval2d<T>(Cj, g.pc, cl.rI, cl.x, cl.uI, cl.y);
-      } else if (cl.kind == 2) {
-        const int L = __ldg(ch_len + cl.ch);
-        v = ch_val[__ldg(ch_start + cl.ch) + ndrift % L];
-      }
-      f[cell] = v;
-      acc2 += (double)((T)__ldg(mt.bu + u) * v);
-    }
-  }
-  // every box must have landed before the block's shared memory is released
-  if (tid == 0) {
-    for (int c = 0; c < nch; ++c)
-      if (!mbar_wait_bounded(&bar[c], 0u)) atomicOr(err, 2u);
-  }
-  red[w][lane] = acc;
-  __syncthreads();
-  if (w == 0 && col_ok) {
-    double sum = 0.0;
-#pragma unroll
-    for (int k = 0; k < NW; ++k) sum += red[k][lane];
-    partial[(size_t)j * g.nr + r] = __ldg(mt.wj + j) * sum;
-  }
-  if (xblock) {
-    // fixed-order reduction of the last column's terms over the block
-    __syncthreads();
-    red[w][lane] = acc2;
-    __syncthreads();
-    if (tid == 0) {
-      double sum = 0.0;
-      for (int k = 0; k < NW; ++k)
-        for (int l = 0; l < 32; ++l) sum += red[k][l];
-      partial[(size_t)j * g.nr + r0 + 32] = __ldg(mt.wj + j) * sum;
-    }
-  }
+  if (!list && threadIdx.x == 0) count[blockIdx.x] = n;
 }
 
-// Strip layouts (the DRIFT_* kinds): DRIFT_STRIP2, 48 columns, 16 warps, two
-// blocks per SM; DRIFT_STRIP1, 48 columns, 32 warps, one block per SM;
-// DRIFT_WINDOW: none, the windowed kernel.  `want` != DRIFT_AUTO asks for
-// one kind, returned only if it fits (else DRIFT_WINDOW).  The default for
-// FP32 storage is DRIFT_STRIP2 where it fits (4 % faster than per-cell box
-// waits on the 513 x 513 x 256 case: the other block on the SM computes while
-// this one's strip lands), else DRIFT_STRIP1 (strips of up to 1028 rows:
-// 14 % faster than the windowed drift on 1025 x 1025 x 512), else the
-// windowed kernel; FP64 takes the windowed kernel (its strips fit one block
-// per SM only, which measured slower).
-template <typename T>
-int drift_strip_width(int nu, int want) {
-  const int nch = (nu + 3 + DS_ROWS - 1) / DS_ROWS;
-  if (nch > 32 || want == DRIFT_WINDOW) return DRIFT_WINDOW;
-  auto dyn = [&](int wc) { return (size_t)nch * (DS_ROWS * wc * sizeof(T) + sizeof(uint64_t)); };
-  // 228 KB of shared memory per SM, 1 KB of it reserved per block; at most
-  // 227 KB per block; static reduction array NW x 32 doubles
-  const bool fit2 = 2 * (dyn(48) + 16 * 32 * 8 + 1024) <= 233472;
-  const bool fit1 = dyn(48) + 32 * 32 * 8 <= 232448;
-  if (want == DRIFT_STRIP2) return fit2 ? DRIFT_STRIP2 : DRIFT_WINDOW;
-  if (want == DRIFT_STRIP1) return fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
-  if (sizeof(T) != 4) return DRIFT_WINDOW;
-  return fit2 ? DRIFT_STRIP2 : fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
+cudaError_t launch_trip_kinds(const uint2 *fp2, uint8_t *kinds, int nr, int nu, int nj,
+                              cudaStream_t st) {
+  const size_t n = trip_kinds_bytes(nr, nu, nj);
+  trip_kind_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(fp2, kinds, nr, nu, nj);
+  return cudaGetLastError();
 }
-
-template <typename T, int WC, int NW, int MINB, int PF = 2>
-static cudaError_t drift_strip_go(const CUtensorMap *tmS, const T *C, T *f, const int32_t *idx,
-                                  const T *fx, const T *fy, const uint2 *fp2,
-                                  const int64_t *ch_start, const int32_t *ch_len,
-                                  const T *ch_val, int64_t ndrift, const MomentTables &mt,
-                                  double *partial, unsigned int *err, uint32_t spins,
-                                  const Geometry &g, cudaStream_t st) {
-  const int nch = (g.nu + 3 + DS_ROWS - 1) / DS_ROWS;
-  const size_t smem = (size_t)nch * DS_ROWS * WC * sizeof(T) + nch * sizeof(uint64_t);
-  cudaError_t e = cudaFuncSetAttribute(drift_strip_kernel<T, WC, NW, MINB, PF>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  // N_r = 32 k + 1 (every grid of the form 2^n + 1): k blocks, the last one
-  // also takes the last column; 2.4 % faster than a block of one column on
-  // the 513 x 513 x 256 case
-  const int extra = (g.nr % 32 == 1 && g.nr > 32) ? 1 : 0;
-  const dim3 grid(extra ? g.nr / 32 : (g.nr + 31) / 32, g.nb);
-  drift_strip_kernel<T, WC, NW, MINB, PF><<<grid, 32 * NW, smem, st>>>(
-      *tmS, C, f, idx, fx, fy, fp2, ch_start, ch_len, ch_val, ndrift, mt, partial, err, spins,
-      extra, g);
+cudaError_t launch_far_cells(const uint2 *fp2, const uint32_t *base, uint32_t *count,
+                             uint32_t *list, int nr, int nu, int nj, cudaStream_t st) {
+  far_cells_kernel<<<nj, 1024, 0, st>>>(fp2, base, count, list, nr, nu);
   return cudaGetLastError();
 }
 
+// The 4 x 4 taps of one cell of a regular trip, in four row slots: at row K
+// of the trip tap row a sits in slot (K + a) & 3, so that the next row drops
+// the first tap row and loads one new one, into slot (K + 3) & 3.  A slot
+// holds the row's second tap and the other three taps' differences from it,
+// formed once when the row is loaded.
+struct TapWin {
+  float b[4], d0[4], d2[4], d3[4];
+  template <int S>
+  __device__ __forceinline__ void row(const float *p) {
+    const float c = p[1];
+    b[S & 3] = c;
+    d0[S & 3] = p[0] - c;
+    d2[S & 3] = p[2] - c;
+    d3[S & 3] = p[3] - c;
+  }
+  // Difference form (see gather_f32x2) about c, the second tap of the second
+  // row: c + sum_a wy_a (b_a - c + sum_{m != 1} wx_m d_am); the x weight of
+  // column 1 is not needed because each direction's weights sum to 1, and
+  // every rounding but the last acts on differences.  Weights / 6, both
+  // directions pairwise: w0 = s^3/6, w3 = t^3/6, w2 = 1/6 + t/2 + t^2/2 -
+  // t^3/2, w1 = w2 at s (s = 1 - t).
+  template <int K>
+  __device__ __forceinline__ float eval(float2 t) const {
+    constexpr int S0 = K & 3, S1 = (K + 1) & 3, S2 = (K + 2) & 3, S3 = (K + 3) & 3;
+    constexpr float k6 = 1.f / 6.f;
+    const float2 kk = f2(k6, k6), h = f2(.5f, .5f);
+    const float2 s = __fadd2_rn(f2(1.f, 1.f), f2(-t.x, -t.y));
+    const float2 w3 = __fmul2_rn(__fmul2_rn(t, t), __fmul2_rn(t, kk));
+    const float2 w0 = __fmul2_rn(__fmul2_rn(s, s), __fmul2_rn(s, kk));
+    const float2 w2 = __ffma2_rn(t, __ffma2_rn(t, __ffma2_rn(t, f2(-.5f, -.5f), h), h), kk);
+    const float wy1 = __fmaf_rn(s.y, __fmaf_rn(s.y, __fmaf_rn(s.y, -.5f, .5f), .5f), k6);
+    const float c = b[S1];
+    const float z1 = __fmaf_rn(w3.x, d3[S1], __fmaf_rn(w2.x, d2[S1], w0.x * d0[S1]));
+    const float z0 = __fmaf_rn(
+        w3.x, d3[S0], __fmaf_rn(w2.x, d2[S0], __fmaf_rn(w0.x, d0[S0], b[S0] - c)));
+    const float z2 = __fmaf_rn(
+        w3.x, d3[S2], __fmaf_rn(w2.x, d2[S2], __fmaf_rn(w0.x, d0[S2], b[S2] - c)));
+    const float z3 = __fmaf_rn(
+        w3.x, d3[S3], __fmaf_rn(w2.x, d2[S3], __fmaf_rn(w0.x, d0[S3], b[S3] - c)));
+    return c + __fmaf_rn(w3.y, z3, __fmaf_rn(w2.y, z2, __fmaf_rn(wy1, z1, w0.y * z0)));
+  }
+};
+
+// Rows [8 t, 8 t + 8) of one strip column per lane.  In a regular trip the
+// taps of row K + 1 are those of row K one coefficient row further down, so a
+// cell loads 4 new taps instead of 16 and needs no index, test or vote; the
+// others test every cell and gather its 16 taps, or read the value of an edge
+// cell.  q: the footpoint words of the trip's first DS_AHEAD rows on entry, of
+// the rows at `pn` on return (in flight that many rows ahead); rows past the
+// slice read the next slice or the tables' padding (FOOT_PAD_ROWS rows).  Returns
+// the trip's moment sum.
+__device__ __forceinline__ double strip_trip(bool regular, const float *win, const float *bu,
+                                             int x0, int rows_left, uint2 (&q)[DS_AHEAD],
+                                             const uint2 *p, const uint2 *pn, float *o,
+                                             uint32_t nr) {
+  static_assert(DS_TRIP <= FOOT_PAD_ROWS, "a trip's loads reach past the padding rows");
+  constexpr int WC = DS_WC;
+  double acc = 0.0;
+  if (regular) {
+    // moment weights of the trip's rows (the table is padded to whole trips)
+    const float4 bl = *reinterpret_cast<const float4 *>(bu);
+    const float4 bh = *(reinterpret_cast<const float4 *>(bu) + 1);
+    const float bk[DS_TRIP] = {bl.x, bl.y, bl.z, bl.w, bh.x, bh.y, bh.z, bh.w};
+    const float *q0 = win + (int)(q[0].y >> FP_FBITS) * WC + ((int)(q[0].x >> FP_FBITS) - x0);
+    TapWin tw;
+    tw.row<0>(q0);
+    tw.row<1>(q0 + WC);
+    tw.row<2>(q0 + 2 * WC);
+    float part = 0.f;
+    p = DS_AHEAD < DS_TRIP ? p + DS_AHEAD * nr : pn;
+#define VLS_REGULAR_ROW(K)                          \
+  {                                                 \
+    const float2 xy = frac21x2(q[(K) % DS_AHEAD]);  \
+    q[(K) % DS_AHEAD] = __ldg(p);                   \
+    p = (K) == DS_TRIP - DS_AHEAD - 1 ? pn : p + nr; \
+    tw.row<(K) + 3>(q0 + ((K) + 3) * WC);           \
+    const float v = tw.eval<K>(xy);                 \
+    *o = v;                                         \
+    o += nr;                                        \
+    if ((K) & 1)                                    \
+      acc += (double)(part + bk[K] * v);            \
+    else                                            \
+      part = bk[K] * v;                             \
+  }
+    VLS_REGULAR_ROW(0)
+    VLS_REGULAR_ROW(1)
+    VLS_REGULAR_ROW(2)
+    VLS_REGULAR_ROW(3)
+    VLS_REGULAR_ROW(4)
+    VLS_REGULAR_ROW(5)
+    VLS_REGULAR_ROW(6)
+    VLS_REGULAR_ROW(7)
+#undef VLS_REGULAR_ROW
+    return acc;
+  }
+#pragma unroll 1
+  for (int k = 0; k < DS_TRIP; k += 2) {
+    const uint2 c[2] = {q[0], q[1]};
+#pragma unroll
+    for (int h = 0; h + 2 < DS_AHEAD; ++h) q[h] = q[h + 2];
+    const int ka = k + DS_AHEAD;  // the rows two words of which are loaded now
+    const uint2 *pp = ka < DS_TRIP ? p + ka * nr : pn + (ka - DS_TRIP) * nr;
+    q[DS_AHEAD - 2] = __ldg(pp);
+    q[DS_AHEAD - 1] = __ldg(pp + nr);
+    float v[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t wc = (c[h].x >> FP_FBITS) - (uint32_t)x0;
+      const bool in = c[h].x < FP_CHAIN && wc < (uint32_t)(WC - 3), row = k + h < rows_left;
+      float edge = 0.f;
+      if (!in && c[h].x != FP_OUT && row) edge = o[h * nr];
+      const float2 xy = frac21x2(c[h]);
+      v[h] = eval_pitch_f32x2<WC>(win + (in ? (c[h].y >> FP_FBITS) * WC + wc : 0u), xy.x, xy.y);
+      v[h] = in ? v[h] : edge;
+      if (row)
+        o[h * nr] = v[h];
+      else
+        v[h] = 0.f;
+    }
+    acc += (double)(bu[k] * v[0] + bu[k + 1] * v[1]);
+    o += 2 * nr;
+  }
+  return acc;
+}
+
+// Shared memory of the strip drift: NB strip buffers (nch boxes of `rows`
+// rows), then per buffer the column sums of every warp and the trips' kinds,
+// then the moment weights.  The boxes hold N_u + 3 rows with as little excess
+// as even heights of at most 256 rows give (16-byte-multiple boxes on
+// 128-byte boundaries).
+struct StripSmem {
+  size_t strip, red, kinds, total;  // bytes: one buffer's parts, everything
+  int nch, rows, nt;
+};
+__host__ __device__ inline StripSmem strip_smem(int nu, int nw, int nb) {
+  StripSmem s;
+  s.nch = (nu + 3 + 255) / 256;
+  s.rows = (nu + 3 + 2 * s.nch - 1) / (2 * s.nch) * 2;
+  s.nt = strip_trips(nu);
+  s.strip = (size_t)s.nch * s.rows * DS_WC * sizeof(float);
+  s.red = ((size_t)nw * 33 * sizeof(double) + 15) / 16 * 16;
+  s.kinds = (size_t)(s.nt + 15) / 16 * 16;
+  s.total = nb * (s.strip + s.red + s.kinds) + (size_t)s.nt * DS_TRIP * sizeof(float);
+  return s;
+}
+int drift_strip_box_rows(int nu) { return strip_smem(nu, 1, 1).rows; }
+
+// Block: NW consumer warps and a producer warp; persistent, a task being one
+// strip (32 output columns) of one J slice.  The producer keeps NB strips
+// staged or in flight: it issues a strip's TMA boxes and fetches its trips'
+// kinds (full barrier); when every consumer is done with a strip (done
+// barrier) it sums their column sums in warp order and refills the buffer
+// with the strip NB tasks later.  The consumers take the strips' trips in
+// turn without a block barrier: a warp that has no more trips in a strip goes
+// on to the next one, so neither the staging of a strip nor the uneven cost
+// of its trips (only the rows near v_r = 0 of the inner columns gather at
+// all) leaves the SM idle.  Which warp takes which trip depends on (strip,
+// slice) alone, and every sum is taken in a fixed order, so the moments do
+// not depend on the grid or the batching.
+//
+// What bounds it: about 60 instructions per cell in regular trips and 110 in
+// the others at some 60 % of the issue slots, and a quarter of the time waits
+// for a strip.  A block per strip with 16 x 2 warps per SM, every cell with
+// its 16 taps and the rare cells gathered in place, took 0.309 ms on the 513 x
+// 513 x 256 Hernquist case, 0.372 on 1025 x 1025 x 64 PLDF and 0.057 on 257 x
+// 257 x 128 Plummer (116 instructions per cell); this form 0.258, 0.305 and
+// 0.049, and edge_kernel 0.012, 0.018 and 0.000 more than the tails alone.
+//
+// Waits are bounded.  A consumer whose wait for a strip ran out (`spins`
+// polls) gathers that strip's cells from global memory; the producer waits
+// (full limit) for a strip's own boxes before it refills its buffer and
+// before the block ends, whatever the consumers did.
+template <int NW, int NB, int MINB>
+__global__ void __launch_bounds__(32 * (NW + 1), MINB)
+    drift_strip_kernel(const __grid_constant__ CUtensorMap tmS, const float *__restrict__ C,
+                       float *f, const uint2 *__restrict__ fp2,
+                       const uint8_t *__restrict__ trip_kinds, MomentTables mt,
+                       double *__restrict__ partial, unsigned int *err, uint32_t spins,
+                       Geometry g) {
+  constexpr int WC = DS_WC;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ uint64_t full[NB], done[NB];
+  const StripSmem L = strip_smem(g.nu, NW, NB);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int ns = strip_blocks(g.nr), ntask = ns * g.nb, nt = L.nt;
+  const bool extra = ns * 32 < g.nr;  // the last strip also takes the last column
+  unsigned char *kinds0 = smem_raw + NB * (L.strip + L.red);
+  float *bus = reinterpret_cast<float *>(kinds0 + NB * L.kinds);
+  auto buf_win = [&](int b) { return reinterpret_cast<float *>(smem_raw + b * L.strip); };
+  auto buf_red = [&](int b) {
+    return reinterpret_cast<double *>(smem_raw + NB * L.strip + b * L.red);
+  };
+  if (tid == 0) {
+    for (int b = 0; b < NB; ++b) {
+      mbar_init(&full[b], 2);  // the boxes, and the kinds
+      mbar_init(&done[b], NW);
+    }
+    mbar_fence_init();
+  }
+  for (int u = tid; u < nt * DS_TRIP; u += 32 * (NW + 1)) bus[u] = __ldg(mt.bu32 + u);
+  __syncthreads();
+  const int nmine = (int)blockIdx.x < ntask ? (ntask - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+
+  if (w == NW) {  // ------------------------------------------------ producer
+    // a strip's boxes; then its trips' kinds (into registers, then into the
+    // buffer), and its share of its slice's footpoint words into L2, where
+    // the trips find them a strip or two later, in flight DS_AHEAD rows ahead
+    auto issue = [&](int i) {
+      const int task = (int)blockIdx.x + i * (int)gridDim.x, b = i % NB;
+      const int jl = task / ns, sx = task - jl * ns;
+      if (lane == 0) {
+        mbar_expect_tx(&full[b], (uint32_t)L.strip);
+        for (int c = 0; c < L.nch; ++c)
+          tma_load_3d(buf_win(b) + (size_t)c * L.rows * WC, &tmS, sx * 32 - DS_XL, c * L.rows, jl,
+                      &full[b]);
+      }
+      __syncwarp();
+    };
+    // into L2 only for strips of up to 352 rows: then the words, coefficients
+    // and values of the strips in flight on the whole chip stay well inside
+    // it (drift 257 x 257 x 128 0.0486 ms with, 0.0523 without; 395 x 307 x
+    // 77 0.0537 and 0.0552; 513 x 513 x 256 0.261 and 0.257; 1025 x 1025 x 64
+    // 0.316 and 0.305)
+    const bool l2_words = g.nu <= 352;
+    constexpr int KPL = 5;  // kinds per lane: strips of up to 1280 rows
+    uint8_t kd[KPL];
+    auto fetch = [&](int i) {
+      const int task = (int)blockIdx.x + i * (int)gridDim.x;
+      const int jl = task / ns, sx = task - jl * ns;
+      const uint8_t *src = trip_kinds + ((size_t)(g.j0 + jl) * ns + sx) * nt;
+#pragma unroll
+      for (int k = 0; k < KPL; ++k) kd[k] = lane + 32 * k < nt ? __ldg(src + lane + 32 * k) : 0;
+    };
+    auto words_to_l2 = [&](int i) {
+      const int task = (int)blockIdx.x + i * (int)gridDim.x;
+      const int jl = task / ns, sx = task - jl * ns;
+      const uint64_t lo = (uint64_t)(g.j0 + jl) * g.nu * g.nr * 8u;
+      const uint64_t n = (uint64_t)g.nu * g.nr * 8u, part = (n / (ns * 32u) + 31u) & ~15ull;
+      const uint64_t at = (uint64_t)(sx * 32 + lane) * part;
+      if (at < n)
+        bulk_prefetch_l2(reinterpret_cast<const char *>(fp2) + ((lo + at) & ~15ull),
+                         (uint32_t)part);
+    };
+    auto kinds_in = [&](int b) {
+#pragma unroll
+      for (int k = 0; k < KPL; ++k)
+        if (lane + 32 * k < nt) kinds0[b * L.kinds + lane + 32 * k] = kd[k];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[b]);
+    };
+    int issued = 0;
+    for (; issued < NB && issued < nmine; ++issued) {
+      issue(issued);
+      fetch(issued);
+      kinds_in(issued % NB);
+      if (l2_words && issued) words_to_l2(issued);
+    }
+    for (int i = 0; i < nmine; ++i) {
+      const int b = i % NB;
+      const uint32_t par = (uint32_t)(i / NB) & 1u;
+      const bool refill = issued < nmine;
+      if (refill) fetch(issued);
+      const bool landed = mbar_wait_idle(&full[b], par);
+      const bool finished = mbar_wait_idle(&done[b], par);
+      if (!__all_sync(0xffffffffu, landed && finished)) {
+        // nothing more is staged; the loads in flight are awaited
+        if (lane == 0) atomicOr(err, 2u);
+        for (int k = i + 1; k < issued; ++k) mbar_wait_idle(&full[k % NB], (uint32_t)(k / NB) & 1u);
+        break;
+      }
+      if (refill) {
+        fence_proxy_async();
+        issue(issued);
+      }
+      const int task = (int)blockIdx.x + i * (int)gridDim.x;
+      const int jl = task / ns, sx = task - jl * ns, j = g.j0 + jl;
+      const double *red = buf_red(b);
+      double sum = 0.0, sumx = 0.0;
+#pragma unroll 8
+      for (int k = 0; k < NW; ++k) sum += red[k * 32 + lane];
+      if (extra && sx == ns - 1 && lane == 0)
+        for (int k = 0; k < NW; ++k) sumx += red[NW * 32 + k];
+      __syncwarp();
+      // the buffer's sums are read: its next strip may complete
+      if (refill) {
+        kinds_in(b);
+        if (l2_words) words_to_l2(issued);
+        ++issued;
+      }
+      const double wj = __ldg(mt.wj + j);
+      if (sx * 32 + lane < g.nr) partial[(size_t)j * g.nr + sx * 32 + lane] = wj * sum;
+      if (extra && sx == ns - 1 && lane == 0)
+        partial[(size_t)j * g.nr + sx * 32 + 32] = wj * sumx;
+    }
+    return;
+  }
+
+  // ----------------------------------------------------------------- consumer
+  const uint32_t nr = (uint32_t)g.nr;
+  uint2 q[DS_AHEAD];
+  auto load_q = [&](const uint2 *p) {
+#pragma unroll
+    for (int k = 0; k < DS_AHEAD; ++k) q[k] = __ldg(p + k * nr);
+  };
+  // this warp's first trip of task i
+  auto first_trip = [&](int task) {
+    const int jl = task / ns;
+    const uint32_t o = (uint32_t)(((uint64_t)(g.j0 + jl) * ns + (task - jl * ns)) * nt % NW);
+    return (int)((w + NW - o) % NW);
+  };
+  auto words = [&](int task, int t) {
+    const int jl = task / ns, sx = task - jl * ns;
+    return fp2 + ((size_t)(g.j0 + jl) * g.nu + DS_TRIP * t) * nr +
+           min(sx * 32 + lane, g.nr - 1);
+  };
+  int task = (int)blockIdx.x;
+  if (nmine > 0) {
+    load_q(words(task, min(first_trip(task), nt - 1)));
+  }
+  for (int i = 0; i < nmine; ++i) {
+    const int b = i % NB;
+    const int jl = task / ns, sx = task - jl * ns, j = g.j0 + jl;
+    const int x0 = sx * 32 - DS_XL;
+    const int tnext = (int)(task + (int)gridDim.x);
+    const float *win = buf_win(b);
+    const unsigned char *kinds = kinds0 + b * L.kinds;
+    const bool ok = __all_sync(
+        0xffffffffu, mbar_wait_idle(&full[b], (uint32_t)(i / NB) & 1u, spins));
+    if (!ok && lane == 0) atomicOr(err, 1u);
+    const uint2 *ws = words(task, 0);
+    float *os = f + (size_t)j * g.nu * nr + min(sx * 32 + lane, g.nr - 1);
+    double acc = 0.0;
+    int t = first_trip(task);
+    if (!ok) {
+      // not staged in time (nor are its kinds): from global memory
+      const float *Cj = C + (size_t)jl * (g.nu + 3) * g.pc;
+      for (; t < nt; t += NW)
+        for (int u = DS_TRIP * t; u < min(DS_TRIP * (t + 1), g.nu); ++u) {
+          RawCell<float> c;
+          c.w = __ldg(ws + (size_t)u * nr);
+          const Cell<float> cl = decode(c);
+          float v = 0.f;
+          if (cl.kind == 0)
+            v = eval2d<float>(Cj, g.pc, cl.rI, cl.x, cl.uI, cl.y);
+          else if (cl.kind == 2)
+            v = os[(size_t)u * nr];
+          os[(size_t)u * nr] = v;
+          acc += (double)(__ldg(mt.bu32 + u) * v);
+        }
+    }
+    bool loaded = true;  // q holds trip t's words (if there is one)
+    bool ahead = false;  // q holds the next strip's first words
+    while (t < nt) {
+      const unsigned char kd = kinds[t];
+      float *o = os + (size_t)(DS_TRIP * t) * nr;
+      const int left = g.nu - DS_TRIP * t;
+      if (kd == TRIP_EMPTY) {
+        const int n = min(DS_TRIP, left);
+        for (int k = 0; k < n; ++k) {
+          *o = 0.f;
+          o += nr;
+        }
+        t += NW;
+        loaded = false;
+        continue;
+      }
+      const uint2 *p = ws + (size_t)(DS_TRIP * t) * nr;
+      if (!loaded) load_q(p);
+      // the words after this trip's: the next trip's, or the next strip's
+      const int t2 = t + NW;
+      const bool more = t2 < nt && kinds[t2] != TRIP_EMPTY;
+      const uint2 *pn = more ? p + (size_t)(DS_TRIP * NW) * nr
+                        : i + 1 < nmine && t2 >= nt
+                            ? words(tnext, min(first_trip(tnext), nt - 1))
+                            : p;
+      acc += strip_trip(kd == TRIP_REGULAR, win, bus + DS_TRIP * t, x0, left, q, p, pn, o, nr);
+      loaded = more;
+      ahead = t2 >= nt;
+      t = t2;
+    }
+    double acc2 = 0.0;
+    if (extra && sx == ns - 1) {
+      // the last column (the strip's columns r0 - 8 .. r0 + 39 cover it), one
+      // row per thread
+      const int rx = sx * 32 + 32;
+      for (int u = w * 32 + lane; u < g.nu; u += 32 * NW) {
+        const size_t cell = ((size_t)j * g.nu + u) * nr + rx;
+        const uint2 c = __ldg(fp2 + cell);
+        float v = 0.f;
+        if (ok && in_strip(c, x0))
+          v = eval_pitch_f32x2<WC>(
+              win + (c.y >> FP_FBITS) * WC + ((c.x >> FP_FBITS) - (uint32_t)x0), frac21(c.x),
+              frac21(c.y));
+        else if (c.x < FP_CHAIN)
+          v = eval2d<float>(C + (size_t)jl * (g.nu + 3) * g.pc, g.pc, (int)(c.x >> FP_FBITS),
+                            frac21(c.x), (int)(c.y >> FP_FBITS), frac21(c.y));
+        else if (c.x == FP_CHAIN)
+          v = f[cell];
+        f[cell] = v;
+        acc2 += (double)(__ldg(mt.bu32 + u) * v);
+      }
+      for (int d = 16; d > 0; d >>= 1) acc2 += __shfl_down_sync(0xffffffffu, acc2, d);
+    }
+    // a strip not awaited above: the producer is done with this buffer's sums
+    // of NB tasks ago only once this task's boxes are in
+    if (!ok && !__all_sync(0xffffffffu, mbar_wait_idle(&full[b], (uint32_t)(i / NB) & 1u)))
+      return;
+    double *red = buf_red(b);
+    red[w * 32 + lane] = acc;
+    if (lane == 0) red[NW * 32 + w] = acc2;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&done[b]);
+    if (!ahead && i + 1 < nmine) {
+      load_q(words(tnext, min(first_trip(tnext), nt - 1)));
+    }
+    task = tnext;
+  }
+}
+
+// Strip layouts (the DRIFT_* kinds), FP32 storage: DRIFT_STRIP2, two strip
+// buffers per block; DRIFT_STRIP1, one (strips too tall for two);
+// DRIFT_WINDOW: none, the windowed kernel.  `want` != DRIFT_AUTO asks for
+// one kind, returned only if it fits (else DRIFT_WINDOW).  FP64 takes the
+// windowed kernel.
 template <typename T>
-cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const T *C, T *f,
-                               const int32_t *idx, const T *fx, const T *fy, const uint2 *fp2,
-                               const int64_t *ch_start, const int32_t *ch_len,
-                               const T *ch_val, int64_t ndrift, const MomentTables &mt,
-                               double *partial, unsigned int *err, uint32_t spins,
-                               const Geometry &g, cudaStream_t st) {
+int drift_strip_width(int nu, int want) {
+  if (sizeof(T) != 4 || want == DRIFT_WINDOW) return DRIFT_WINDOW;
+  // 227 KB of shared memory per block, the barriers' 1 KB kept free
+  const bool fit2 = strip_smem(nu, STRIP_WARPS, 2).total + 1024 <= 232448;
+  const bool fit1 = strip_smem(nu, STRIP_WARPS, 1).total + 1024 <= 232448;
+  if (want == DRIFT_STRIP2) return fit2 ? DRIFT_STRIP2 : DRIFT_WINDOW;
+  if (want == DRIFT_STRIP1) return fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
+  return fit2 ? DRIFT_STRIP2 : fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
+}
+
+template <int NW, int NB, int MINB>
+static cudaError_t drift_strip_go(const CUtensorMap *tmS, const float *C, float *f,
+                                  const uint2 *fp2, const uint8_t *trip_kinds,
+                                  const MomentTables &mt, double *partial, unsigned int *err,
+                                  uint32_t spins, const Geometry &g, cudaStream_t st) {
+  const size_t smem = strip_smem(g.nu, NW, NB).total;
+  cudaError_t e = cudaFuncSetAttribute(drift_strip_kernel<NW, NB, MINB>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  int dev = 0, nsm = 0;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+    return e;
+  const int ntask = strip_blocks(g.nr) * g.nb;
+  drift_strip_kernel<NW, NB, MINB><<<std::min(ntask, nsm * MINB), 32 * (NW + 1), smem, st>>>(
+      *tmS, C, f, fp2, trip_kinds, mt, partial, err, spins, g);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C, float *f,
+                               const uint2 *fp2, const uint8_t *trip_kinds,
+                               const MomentTables &mt, double *partial, unsigned int *err,
+                               uint32_t spins, const Geometry &g, cudaStream_t st) {
   switch (kind) {
     case DRIFT_STRIP2:
-      return drift_strip_go<T, 48, 16, 2>(tmS, C, f, idx, fx, fy, fp2, ch_start, ch_len,
-                                          ch_val, ndrift, mt, partial, err, spins, g, st);
+      return drift_strip_go<STRIP_WARPS, 2, 1>(tmS, C, f, fp2, trip_kinds, mt, partial, err,
+                                               spins, g, st);
     case DRIFT_STRIP1:
-      return drift_strip_go<T, 48, 32, 1>(tmS, C, f, idx, fx, fy, fp2, ch_start, ch_len,
-                                          ch_val, ndrift, mt, partial, err, spins, g, st);
+      return drift_strip_go<STRIP_WARPS, 1, 1>(tmS, C, f, fp2, trip_kinds, mt, partial, err,
+                                               spins, g, st);
     default:
       return cudaErrorInvalidValue;
   }
 }
 
-template <typename T>
-__global__ void chain_tail_kernel(const T *__restrict__ C, T *__restrict__ ch_val,
-                                  const int64_t *__restrict__ ch_start,
-                                  const int32_t *__restrict__ ch_len,
-                                  const int32_t *__restrict__ t_idx,
-                                  const double *__restrict__ t_x,
-                                  const double *__restrict__ t_y,
-                                  const int32_t *__restrict__ t_j, int64_t c_lo,
-                                  int64_t c_hi, int64_t ndrift, Geometry g) {
-  const int64_t c = c_lo + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= c_hi) return;
-  const int L = ch_len[c];
-  const int code = t_idx[c];
-  T v = T(0);
-  if (code >= 0) {
-    const T *Cj = C + (size_t)(t_j[c] - g.j0) * (g.nu + 3) * g.pc;
-    v = eval2d<T>(Cj, g.pc, code & 0xffff, (T)t_x[c], code >> 16, (T)t_y[c]);
+// ------------------------------------------------------------- edge cells
+// One thread per chain (slice jl: chains [chain_lo[j], chain_lo[j + 1])) and,
+// for the strip drift (EDGE), per far-tap cell of the slice.
+//
+// Chain: the spline value at its tail goes into the ring slot that becomes
+// the tail, and, for the strip drift, the front of the ring, this drift's
+// value of the chain's cell, into f; a chain of one element has its tail as
+// front.  The front is loaded before the tail's gather, so that the two
+// latencies overlap.  (The windowed drift reads the fronts itself: 0.010 ms
+// less here, nothing there, on 513 x 513 x 128 in FP64.)
+template <typename T, bool EDGE>
+__global__ void __launch_bounds__(256)
+    edge_kernel(const T *__restrict__ C, T *__restrict__ f, T *__restrict__ ch_val,
+                const int64_t *__restrict__ ch_start, const int32_t *__restrict__ ch_len,
+                const uint32_t *__restrict__ ch_at, const int32_t *__restrict__ t_idx,
+                const double *__restrict__ t_x, const double *__restrict__ t_y,
+                const int32_t *__restrict__ chain_lo, int64_t ndrift,
+                const uint32_t *__restrict__ far_base, const uint32_t *__restrict__ far,
+                const uint2 *__restrict__ fp2, Geometry g) {
+  const int jl = blockIdx.y, j = g.j0 + jl;
+  const T *Cj = C + (size_t)jl * (g.nu + 3) * g.pc;
+  const size_t sb = (size_t)j * g.nu * g.nr;
+  int e = blockIdx.x * 256 + threadIdx.x;
+  const int c = __ldg(chain_lo + j) + e, hi = __ldg(chain_lo + j + 1);
+  if (c < hi) {
+    const int32_t L = __ldg(ch_len + c), code = __ldg(t_idx + c);
+    T *ring = ch_val + __ldg(ch_start + c);
+    // 32-bit remainder of the drift count
+    const uint32_t at = ndrift <= 0xffffffffll ? (uint32_t)ndrift % (uint32_t)L
+                                               : (uint32_t)(ndrift % L);
+    const T front = EDGE ? ring[at] : T(0);
+    T v = T(0);
+    if (code >= 0)
+      v = eval2d<T>(Cj, g.pc, code & 0xffff, (T)__ldg(t_x + c), code >> 16, (T)__ldg(t_y + c));
+    ring[at == 0 ? L - 1 : at - 1] = v;
+    if (EDGE) f[sb + __ldg(ch_at + c)] = L == 1 ? v : front;
+    return;
   }
-  ch_val[ch_start[c] + (ndrift + L - 1) % L] = v;
+  if constexpr (EDGE) {
+    e -= hi - __ldg(chain_lo + j);
+    const uint32_t k = __ldg(far_base + j) + (uint32_t)e;
+    if (k >= __ldg(far_base + j + 1)) return;
+    const size_t cell = sb + __ldg(far + k);
+    RawCell<float> w;
+    w.w = __ldg(fp2 + cell);
+    const Cell<float> cl = decode(w);
+    f[cell] = eval2d<float>(Cj, g.pc, cl.rI, cl.x, cl.uI, cl.y);
+  }
 }
 
+// most: the largest number of edge cells in a slice of this launch
 template <typename T>
-cudaError_t launch_chain_tails(const T *C, T *ch_val, const int64_t *ch_start,
-                               const int32_t *ch_len, const int32_t *t_idx,
-                               const double *t_x, const double *t_y,
-                               int64_t nchains, int64_t c_lo, int64_t c_hi,
-                               int64_t ndrift, const Geometry &g, cudaStream_t st) {
-  if (c_hi <= c_lo) return cudaSuccess;
-  // t_j (slice of each chain) is stored right after t_idx
-  const int32_t *t_j = t_idx + nchains;
-  const int threads = 256;
-  const unsigned blocks = (unsigned)((c_hi - c_lo + threads - 1) / threads);
-  chain_tail_kernel<T><<<blocks, threads, 0, st>>>(C, ch_val, ch_start, ch_len, t_idx,
-                                                   t_x, t_y, t_j, c_lo, c_hi, ndrift, g);
-  return cudaGetLastError();
+cudaError_t launch_edge(const T *C, T *f, T *ch_val, const EdgeTables &t, int64_t ndrift,
+                        const uint2 *fp2, int most, const Geometry &g, cudaStream_t st) {
+  if (most <= 0) return cudaSuccess;
+  auto go = [&](auto kern) {
+    kern<<<dim3((most + 255) / 256, g.nb), 256, 0, st>>>(
+        C, f, ch_val, t.ch_start, t.ch_len, t.ch_at, t.t_idx, t.t_x, t.t_y, t.chain_lo, ndrift,
+        t.far_base, t.far, fp2, g);
+    return cudaGetLastError();
+  };
+  if constexpr (sizeof(T) == 4)
+    if (t.far_base) return go(edge_kernel<T, true>);
+  return go(edge_kernel<T, false>);
 }
 
 // ------------------------------------------------------------------ moment
@@ -1502,20 +1728,13 @@ cudaError_t launch_nonfinite(const T *f, size_t n, unsigned int *flag,
 
 #define VLS_INST(T)                                                            \
   template int drift_strip_width<T>(int, int);                                  \
-  template cudaError_t launch_drift_strip<T>(                                   \
-      const CUtensorMap *, int, const T *, T *, const int32_t *, const T *, const T *, \
-      const uint2 *, const int64_t *, const int32_t *, const T *, int64_t,       \
-      const MomentTables &, double *, unsigned int *, uint32_t, const Geometry &, \
-      cudaStream_t);                                                            \
   template cudaError_t launch_drift_tma<T>(                                     \
       const CUtensorMap *, const T *, T *, const int32_t *, const T *, const T *, \
       const uint2 *, const int64_t *, const int32_t *, const T *, int64_t,        \
       const MomentTables &, double *, unsigned int *, uint32_t, const Geometry &, \
       cudaStream_t);                                                            \
-  template cudaError_t launch_chain_tails<T>(                                   \
-      const T *, T *, const int64_t *, const int32_t *, const int32_t *,         \
-      const double *, const double *, int64_t, int64_t, int64_t, int64_t,       \
-      const Geometry &, cudaStream_t);                                          \
+  template cudaError_t launch_edge<T>(const T *, T *, T *, const EdgeTables &, int64_t, \
+                                      const uint2 *, int, const Geometry &, cudaStream_t); \
   template cudaError_t launch_moment<T>(const T *, const MomentTables &,        \
                                         double *, const Geometry &,             \
                                         cudaStream_t);                          \
