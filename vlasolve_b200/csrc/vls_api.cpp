@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/vlasolve_b200.h"
+#include "vls_hostcopy.h"
 #include "vls_internal.h"
 #include "vls_setup.h"
 
@@ -62,6 +63,7 @@ struct vls_handle {
   unsigned int *count = nullptr, *flag = nullptr;
   double *stats_part = nullptr;
   size_t stats_nblk = 0;
+  HostCopy copy;  // large pageable host arrays
   double *staging = nullptr;
   size_t staging_n = 0;
   // host copies of the chain layout
@@ -185,7 +187,7 @@ static int dalloc(vls_handle *h, P **p, size_t bytes) {
 }
 
 static int upload(vls_handle *h, void *dst, const void *src, size_t bytes) {
-  CK(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->st));
+  CK(h, h->copy.upload(dst, src, bytes, h->st));
   CK(h, cudaStreamSynchronize(h->st));
   return VLS_OK;
 }
@@ -420,7 +422,8 @@ static int encode_and_upload_footpoints(vls_handle *h, bool build_chains) {
       TRY(upload(h, (double *)h->fx + off, fx.data(), n * sizeof(double)));
       TRY(upload(h, (double *)h->fy + off, fy.data(), n * sizeof(double)));
     } else {
-      for (size_t i = 0; i < n; i++) packed[i] = encode_packed(c, idx[i], fx[i], fy[i]);
+#pragma omp parallel for
+      for (int64_t i = 0; i < (int64_t)n; i++) packed[i] = encode_packed(c, idx[i], fx[i], fy[i]);
       TRY(upload(h, h->fp2 + off, packed.data(), n * sizeof(uint2)));
     }
   }
@@ -599,6 +602,7 @@ static void free_all(vls_handle *h) {
   }
   if (h->ev_fork) cudaEventDestroy(h->ev_fork);
   h->ev_fork = nullptr;
+  h->copy.release();
   if (h->st) cudaStreamDestroy(h->st);
   h->st = nullptr;
 }
@@ -866,13 +870,11 @@ static int check_device_flags(vls_handle *h);
 // ------------------------------------------------------------- f transfer
 static int put_f(vls_handle *h, const double *host) {
   if (h->prec == VLS_FP64) {
-    CK(h, cudaMemcpyAsync(h->f, host, sizeof(double) * h->cells,
-                          cudaMemcpyHostToDevice, h->st));
+    CK(h, h->copy.upload(h->f, host, sizeof(double) * h->cells, h->st));
   } else {
     for (size_t off = 0; off < h->cells; off += h->staging_n) {
       const size_t n = std::min(h->staging_n, h->cells - off);
-      CK(h, cudaMemcpyAsync(h->staging, host + off, sizeof(double) * n,
-                            cudaMemcpyHostToDevice, h->st));
+      CK(h, h->copy.upload(h->staging, host + off, sizeof(double) * n, h->st));
       CK(h, timed(h, VLS_K_CONVERT, [&] {
            return launch_convert_in<float>(h->staging, (float *)h->f + off, n, h->st);
          }));
@@ -890,8 +892,7 @@ static int put_f(vls_handle *h, const double *host) {
 
 static int take_f(vls_handle *h, double *host) {
   if (h->prec == VLS_FP64) {
-    CK(h, cudaMemcpyAsync(host, h->f, sizeof(double) * h->cells,
-                          cudaMemcpyDeviceToHost, h->st));
+    CK(h, h->copy.download(host, h->f, sizeof(double) * h->cells, h->st));
   } else {
     for (size_t off = 0; off < h->cells; off += h->staging_n) {
       const size_t n = std::min(h->staging_n, h->cells - off);
@@ -899,8 +900,7 @@ static int take_f(vls_handle *h, double *host) {
            return launch_convert_out<float>((const float *)h->f + off, h->staging, n,
                                             h->st);
          }));
-      CK(h, cudaMemcpyAsync(host + off, h->staging, sizeof(double) * n,
-                            cudaMemcpyDeviceToHost, h->st));
+      CK(h, h->copy.download(host + off, h->staging, sizeof(double) * n, h->st));
     }
   }
   CK(h, cudaStreamSynchronize(h->st));
@@ -1914,7 +1914,7 @@ static int adjoint_backward_impl(vls_handle *h, const double *dbins, double *df0
   if (b.pending) CK(h, launch_moment_adj(b.lam, b.beta, mt, g, h->st));
   // results: the derivative with respect to the initial grid and the initial
   // chain values (logical ring order at the first step)
-  CK(h, cudaMemcpyAsync(df0, b.lam, cells * sizeof(double), cudaMemcpyDeviceToHost, h->st));
+  CK(h, h->copy.download(df0, b.lam, cells * sizeof(double), h->st));
   std::vector<double> rb((size_t)h->nel);
   if (h->nel)
     CK(h, cudaMemcpyAsync(rb.data(), b.ringb, rb.size() * sizeof(double),

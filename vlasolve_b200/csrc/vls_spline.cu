@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../../include/vlasolve_b200.h"
+#include "vls_hostcopy.h"
 #include "vls_internal.h"
 #include "vls_setup.h"
 
@@ -48,6 +49,7 @@ struct vls_spline2d {
   int rc_cfg[2] = {-1, -1};  // register layouts of the u (dim1) and r (dim0) lines
   RcDir<double> rcd[2];
   bool assigned = false, built = false;
+  HostCopy copy;  // large pageable host arrays
   // point buffers of the gathers (grown on demand)
   void *pts = nullptr;
   size_t pts_bytes = 0;
@@ -93,6 +95,7 @@ void sfree(vls_spline2d *s) {
   s->allocs.clear();
   if (s->pts) cudaFree(s->pts);
   s->pts = nullptr;
+  s->copy.release();
   if (s->st) cudaStreamDestroy(s->st);
   s->st = nullptr;
 }
@@ -260,12 +263,13 @@ extern "C" int vls_spline2d_assign(vls_spline2d *s, const double *data, int64_t 
   SCK(s, cudaSetDevice(s->d.device));
   const size_t n = (size_t)s->dim[0] * s->dim[1] * s->ns;
   if (s->esize == 8) {
-    SCK(s, cudaMemcpyAsync(s->f, data, sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
+    SCK(s, s->copy.upload(s->f, data, sizeof(double) * n, s->st));
     SCK(s, cudaStreamSynchronize(s->st));
   } else {
-    std::vector<float> h(n);
-    for (size_t i = 0; i < n; ++i) h[i] = (float)data[i];
-    SCK(s, cudaMemcpyAsync(s->f, h.data(), sizeof(float) * n, cudaMemcpyHostToDevice, s->st));
+    const std::unique_ptr<float[]> h(new float[n]);
+#pragma omp parallel for if (n > 65536)
+    for (int64_t i = 0; i < (int64_t)n; ++i) h[i] = (float)data[i];
+    SCK(s, s->copy.upload(s->f, h.get(), sizeof(float) * n, s->st));
     SCK(s, cudaStreamSynchronize(s->st));
   }
   s->assigned = true;
@@ -342,6 +346,7 @@ extern "C" int vls_spline2d_pos2coord(const vls_spline2d *sc, int32_t dir, int64
   if (!s || (n > 0 && (!p || !I || !F)))
     return sfail(s, VLS_EINVAL, "vls_spline2d_pos2coord: NULL argument");
   if (dir != 0 && dir != 1) return sfail(s, VLS_EINVAL, "vls_spline2d_pos2coord: dir 0 or 1");
+#pragma omp parallel for if (n > 4096)
   for (int64_t i = 0; i < n; ++i) {
     double ip;
     const double x = std::modf((rescale(p[i], s->d.scaleType[dir]) - s->start[dir]) *
@@ -492,13 +497,19 @@ int run_points(vls_spline2d *s, int mode, int64_t n, const int64_t *slice, const
   if (!s->built) return sfail(s, VLS_ESTATE, "spline evaluated before build");
   if (n < 0) return sfail(s, VLS_EINVAL, "negative point count");
   if (n == 0) return VLS_OK;
+  // the first point outside the nodes or the slices, if any
+  int64_t out = n, outs = n;
+#pragma omp parallel for reduction(min : out, outs) if (n > 4096)
   for (int64_t i = 0; i < n; ++i) {
     if (NX[i] < 0 || NX[i] >= s->dim[0] || NY[i] < 0 || NY[i] >= s->dim[1])
-      return sfail(s, VLS_EINVAL,
-                   "point " + std::to_string(i) + " lies outside the spline's nodes");
-    if (slice && (slice[i] < 0 || slice[i] >= s->ns))
-      return sfail(s, VLS_EINVAL, "point " + std::to_string(i) + ": slice out of range");
+      out = std::min(out, i);
+    if (slice && (slice[i] < 0 || slice[i] >= s->ns)) outs = std::min(outs, i);
   }
+  if (out < n && out <= outs)
+    return sfail(s, VLS_EINVAL,
+                 "point " + std::to_string(out) + " lies outside the spline's nodes");
+  if (outs < n)
+    return sfail(s, VLS_EINVAL, "point " + std::to_string(outs) + ": slice out of range");
   SCK(s, cudaSetDevice(s->d.device));
   const size_t nn = (size_t)n;
   const int nout = mode == EV_HESS ? 7 : mode == EV_GRAD ? 3 : 1;
@@ -520,19 +531,19 @@ int run_points(vls_spline2d *s, int mode, int64_t n, const int64_t *slice, const
   double *d_g = d_v + nn, *d_h = d_v + 3 * nn;
   int32_t *d_nx = (int32_t *)(b + 24 * nn + 8 * nn * (size_t)nout);
   int32_t *d_ny = d_nx + nn;
-  if (slice) SCK(s, cudaMemcpyAsync(d_sl, slice, 8 * nn, cudaMemcpyHostToDevice, s->st));
-  if (mode != EV_NXPY) SCK(s, cudaMemcpyAsync(d_x, X, 8 * nn, cudaMemcpyHostToDevice, s->st));
-  SCK(s, cudaMemcpyAsync(d_y, Y, 8 * nn, cudaMemcpyHostToDevice, s->st));
-  SCK(s, cudaMemcpyAsync(d_nx, NX, 4 * nn, cudaMemcpyHostToDevice, s->st));
-  SCK(s, cudaMemcpyAsync(d_ny, NY, 4 * nn, cudaMemcpyHostToDevice, s->st));
+  if (slice) SCK(s, s->copy.upload(d_sl, slice, 8 * nn, s->st));
+  if (mode != EV_NXPY) SCK(s, s->copy.upload(d_x, X, 8 * nn, s->st));
+  SCK(s, s->copy.upload(d_y, Y, 8 * nn, s->st));
+  SCK(s, s->copy.upload(d_nx, NX, 4 * nn, s->st));
+  SCK(s, s->copy.upload(d_ny, NY, 4 * nn, s->st));
   SCK(s, s->esize == 8 ? launch_points<double>(s, mode, n, d_sl, d_nx, d_x, d_ny, d_y, d_v, d_g,
                                                d_h)
                        : launch_points<float>(s, mode, n, d_sl, d_nx, d_x, d_ny, d_y, d_v, d_g,
                                               d_h));
-  SCK(s, cudaMemcpyAsync(v, d_v, 8 * nn, cudaMemcpyDeviceToHost, s->st));
+  SCK(s, s->copy.download(v, d_v, 8 * nn, s->st));
   if (mode == EV_GRAD || mode == EV_HESS)
-    SCK(s, cudaMemcpyAsync(g, d_g, 16 * nn, cudaMemcpyDeviceToHost, s->st));
-  if (mode == EV_HESS) SCK(s, cudaMemcpyAsync(h, d_h, 32 * nn, cudaMemcpyDeviceToHost, s->st));
+    SCK(s, s->copy.download(g, d_g, 16 * nn, s->st));
+  if (mode == EV_HESS) SCK(s, s->copy.download(h, d_h, 32 * nn, s->st));
   SCK(s, cudaStreamSynchronize(s->st));
   return VLS_OK;
 }
@@ -555,12 +566,12 @@ extern "C" int vls_spline2d_evaluate_nxpy(vls_spline2d *s, int64_t n, const int6
                                           const int32_t *Nx, const double *yy, double *v) {
   if (!s || (n > 0 && (!Nx || !yy || !v)))
     return sfail(s, VLS_EINVAL, "vls_spline2d_evaluate_nxpy: NULL argument");
-  std::vector<int32_t> NY((size_t)std::max<int64_t>(n, 0));
-  std::vector<double> Y(NY.size());
-  const int rc = vls_spline2d_pos2coord(s, 1, n, yy, NY.data(), Y.data());
+  const size_t nn = (size_t)std::max<int64_t>(n, 0);
+  const std::unique_ptr<int32_t[]> NY(new int32_t[nn]);  // written in parallel
+  const std::unique_ptr<double[]> Y(new double[nn]);
+  const int rc = vls_spline2d_pos2coord(s, 1, n, yy, NY.get(), Y.get());
   if (rc != VLS_OK) return rc;
-  return run_points(s, EV_NXPY, n, slice, Nx, nullptr, NY.data(), Y.data(), v, nullptr,
-                    nullptr);
+  return run_points(s, EV_NXPY, n, slice, Nx, nullptr, NY.get(), Y.get(), v, nullptr, nullptr);
 }
 
 // localSpline::evaluate(double, double) (localSpline.hxx:477-488): pos2Coord
@@ -570,13 +581,13 @@ extern "C" int vls_spline2d_evaluate(vls_spline2d *s, int64_t n, const int64_t *
   if (!s || (n > 0 && (!xx || !yy || !v)))
     return sfail(s, VLS_EINVAL, "vls_spline2d_evaluate: NULL argument");
   const size_t nn = (size_t)std::max<int64_t>(n, 0);
-  std::vector<int32_t> NX(nn), NY(nn);
-  std::vector<double> X(nn), Y(nn);
-  int rc = vls_spline2d_pos2coord(s, 0, n, xx, NX.data(), X.data());
-  if (rc == VLS_OK) rc = vls_spline2d_pos2coord(s, 1, n, yy, NY.data(), Y.data());
+  const std::unique_ptr<int32_t[]> NX(new int32_t[nn]), NY(new int32_t[nn]);
+  const std::unique_ptr<double[]> X(new double[nn]), Y(new double[nn]);
+  int rc = vls_spline2d_pos2coord(s, 0, n, xx, NX.get(), X.get());
+  if (rc == VLS_OK) rc = vls_spline2d_pos2coord(s, 1, n, yy, NY.get(), Y.get());
   if (rc != VLS_OK) return rc;
-  return run_points(s, EV_VALUE, n, slice, NX.data(), X.data(), NY.data(), Y.data(), v,
-                    nullptr, nullptr);
+  return run_points(s, EV_VALUE, n, slice, NX.get(), X.get(), NY.get(), Y.get(), v, nullptr,
+                    nullptr);
 }
 
 // ---------------------------------------------------------- interpolSpline
@@ -722,11 +733,12 @@ extern "C" int vls_interp_evaluate(vls_interp *s, int64_t n, const double *x, co
   if (n <= 0) return n < 0 ? ifail(s, VLS_EINVAL, "negative point count") : VLS_OK;
   const vls_interp_init &I = s->ini;
   const size_t nn = (size_t)n;
-  std::vector<int32_t> NX(nn), NY(nn);
-  std::vector<double> X(nn), Y(nn);
+  const std::unique_ptr<int32_t[]> NX(new int32_t[nn]), NY(new int32_t[nn]);
+  const std::unique_ptr<double[]> X(new double[nn]), Y(new double[nn]);
   double st[2], hi[2];
   vls_spline2d_scale(s->sp, st, hi);
-  for (size_t i = 0; i < nn; ++i) {
+#pragma omp parallel for if (nn > 4096)
+  for (int64_t i = 0; i < n; ++i) {
     double px = x[i], py = y[i];
     if (I.rescaleNeeded) {
       px = rescale(px, I.xscaleType);
@@ -741,11 +753,12 @@ extern "C" int vls_interp_evaluate(vls_interp *s, int64_t n, const double *x, co
     NY[i] = std::min((int32_t)ip, I.ny - 1);
   }
   const int mode = h ? EV_HESS : g ? EV_GRAD : EV_VALUE;
-  const int rc = run_points(s->sp, mode, n, nullptr, NX.data(), X.data(), NY.data(), Y.data(),
-                            v, g, h);
+  const int rc =
+      run_points(s->sp, mode, n, nullptr, NX.get(), X.get(), NY.get(), Y.get(), v, g, h);
   if (rc != VLS_OK) return ifail(s, rc, vls_spline2d_last_error(s->sp));
   if (I.useLog)
-    for (size_t i = 0; i < nn; ++i) {
+#pragma omp parallel for if (nn > 4096)
+    for (int64_t i = 0; i < n; ++i) {
       v[i] = std::exp(std::max(v[i], -700.0));
       if (g) {
         g[2 * i] = -g[2 * i] * v[i];
