@@ -62,7 +62,6 @@ struct vls_handle {
          *shift = nullptr, *mtot = nullptr;
   unsigned int *count = nullptr, *flag = nullptr;
   double *stats_part = nullptr;
-  size_t stats_nblk = 0;
   HostCopy copy;  // large pageable host arrays
   double *staging = nullptr;
   size_t staging_n = 0;
@@ -733,14 +732,13 @@ extern "C" int vls_create_layout(const vls_grid_desc *grid, const vls_solver_des
   A(dalloc(hp, &h->Rcoef, sizeof(double) * c.nr));
   A(dalloc(hp, &h->partial, sizeof(double) * (size_t)c.nj * c.nr));
   A(dalloc(hp, &h->T2, sizeof(double) * c.nr));
-  A(dalloc(hp, &h->bins, sizeof(double) * c.nr));
+  A(dalloc(hp, &h->bins, sizeof(double) * (c.nr + 4)));  // and the four integrals of the stats
   A(dalloc(hp, &h->Mr, sizeof(double) * c.nr));
   A(dalloc(hp, &h->shift, sizeof(double) * c.nr));
   A(dalloc(hp, &h->mtot, sizeof(double) * 2));
   A(dalloc(hp, &h->count, sizeof(unsigned int) * 4));
   A(dalloc(hp, &h->flag, sizeof(unsigned int) * 4));
-  h->stats_nblk = (size_t)((c.nu + 7) / 8) * c.nj;
-  A(dalloc(hp, &h->stats_part, sizeof(double) * 8 * h->stats_nblk));
+  A(dalloc(hp, &h->stats_part, sizeof(double) * 8 * stats_blocks(c.nu, c.nj)));
   h->staging_n = std::min<size_t>(cells, (size_t)16 << 20);
   if (h->prec != VLS_FP64) A(dalloc(hp, &h->staging, sizeof(double) * h->staging_n));
   if (s != VLS_OK) {
@@ -884,10 +882,10 @@ static int put_f(vls_handle *h, const double *host) {
   CK(h, h->prec == VLS_FP64
             ? launch_nonfinite<double>((const double *)h->f, h->cells, h->flag + 2, h->st)
             : launch_nonfinite<float>((const float *)h->f, h->cells, h->flag + 2, h->st));
-  CK(h, cudaStreamSynchronize(h->st));
+  const int flags = check_device_flags(h);  // waits for the stream
   h->have_f = true;
   h->moments_valid = false;
-  return check_device_flags(h);
+  return flags;
 }
 
 static int take_f(vls_handle *h, double *host) {
@@ -903,8 +901,7 @@ static int take_f(vls_handle *h, double *host) {
       CK(h, h->copy.download(host + off, h->staging, sizeof(double) * n, h->st));
     }
   }
-  CK(h, cudaStreamSynchronize(h->st));
-  return check_device_flags(h);
+  return check_device_flags(h);  // waits for the stream
 }
 
 extern "C" int vls_set_f(vls_handle *h, const double *host, size_t n) {
@@ -1309,9 +1306,9 @@ static int check_device_flags(vls_handle *h) {
 extern "C" int vls_sync(vls_handle *h) {
   if (!h) return VLS_EINVAL;
   CK(h, cudaSetDevice(h->solver.device));
-  CK(h, cudaStreamSynchronize(h->st));
+  const int flags = check_device_flags(h);  // waits for the stream
   CK(h, cudaGetLastError());
-  return check_device_flags(h);
+  return flags;
 }
 
 extern "C" int vls_kernel_launches(const vls_handle *h, int64_t *n) {
@@ -1395,38 +1392,21 @@ extern "C" int vls_last_mass_async(vls_handle *h, double *mtot) {
 }
 
 // ------------------------------------------------------------------ stats
-static void two_sum_acc(double &s, double &c, double x) {
-  const double t = s + x;
-  const double bb = t - s;
-  c += (s - (t - bb)) + (x - bb);
-  s = t;
-}
-
 template <typename T>
 static int stats_impl(vls_handle *h, vls_stats_out *o) {
   const Coords &c = h->co;
   TRY(moments_impl<T>(h));
-  std::vector<double> bins(c.nr);
-  CK(h, cudaMemcpyAsync(bins.data(), h->bins, sizeof(double) * c.nr,
-                        cudaMemcpyDeviceToHost, h->st));
   CK(h, timed(h, VLS_K_STATS, [&] {
        return launch_stats<T>((const T *)h->f, h->dR_val, h->dU_val, h->dJ_val,
-                              h->d_dR, h->d_dU, h->d_Ct1, h->stats_part, nullptr,
+                              h->d_dR, h->d_dU, h->d_Ct1, h->stats_part, h->bins + c.nr,
                               geometry(h), h->st);
      }));
-  std::vector<double> part(8 * h->stats_nblk);
-  CK(h, cudaMemcpyAsync(part.data(), h->stats_part, sizeof(double) * part.size(),
+  h->launches++;
+  std::vector<double> bins((size_t)c.nr + 4);
+  CK(h, cudaMemcpyAsync(bins.data(), h->bins, sizeof(double) * bins.size(),
                         cudaMemcpyDeviceToHost, h->st));
   CK(h, cudaStreamSynchronize(h->st));
-  double q[4];
-  for (int k = 0; k < 4; k++) {
-    double s = 0, cc = 0;
-    for (size_t b = 0; b < h->stats_nblk; b++) {
-      two_sum_acc(s, cc, part[b * 8 + 2 * k]);
-      two_sum_acc(s, cc, part[b * 8 + 2 * k + 1]);
-    }
-    q[k] = s + cc;
-  }
+  const double *q = bins.data() + c.nr;
   // vlasovSolver21::potentialEnergy (vlasovSolver21.hxx:627-642); the last
   // shell (mass 0) is skipped instead of reading past R_Val
   double M = 0, Ep = 0;

@@ -229,6 +229,8 @@ cudaError_t launch_scan(const double *partial, const MomentTables &mt,
                         double *T2, double *bins, double *Mr, double *shift,
                         double *mtot, unsigned int *count, unsigned int *status,
                         const Geometry &g, cudaStream_t st);
+// Ek, S, L1, L2 into out4 (device); part: 8 doubles per block of the kernel
+size_t stats_blocks(int nu, int nj);
 template <typename T>
 cudaError_t launch_stats(const T *f, const double *R, const double *U,
                          const double *J, const double *dR, const double *dU,
