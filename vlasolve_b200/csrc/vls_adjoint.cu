@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "vls_async.cuh"
 #include "vls_dd.cuh"
 #include "vls_internal.h"
 
@@ -204,6 +205,7 @@ __global__ void ucol_adj_kernel(const T *__restrict__ f, double *__restrict__ Gb
 __global__ void __launch_bounds__(1024) shift_adj_kernel(const double *__restrict__ sbar,
                                                          double *beta, unsigned int *count,
                                                          MomentTables mt, Geometry g) {
+  chain_begin();
   __shared__ double part[32][33];
   __shared__ dd wsum[32];
   __shared__ bool last;
@@ -440,6 +442,7 @@ __global__ void chain_adj_kernel(const double *__restrict__ lam, const double *_
                                  const int64_t *__restrict__ ch_start,
                                  const int32_t *__restrict__ ch_len, int64_t nch,
                                  int64_t ndrift, Geometry g) {
+  chain_begin();
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (c >= nch) return;
   const int L = ch_len[c];
@@ -500,6 +503,7 @@ __global__ void inv_perm_kernel(const uint32_t *__restrict__ ent,
                                 const double *__restrict__ mB, MomentTables mt,
                                 const double *__restrict__ tv, double *__restrict__ vperm,
                                 Geometry g) {
+  chain_begin();
   const int j = blockIdx.y;
   const int64_t e0 = ebase[j], e1 = ebase[j + 1];
   const size_t cbase = (size_t)j * g.nr * g.nu;
@@ -584,6 +588,7 @@ __global__ void __launch_bounds__(128)
                                 const int32_t *__restrict__ t_idx,
                                 const double *__restrict__ t_x, const double *__restrict__ t_y,
                                 Geometry g) {
+  chain_begin();
   const int q0 = (blockIdx.x * 32 + threadIdx.x) * Q;
   const int p0 = (blockIdx.y * blockDim.y + threadIdx.y) * RB;
   const int j = blockIdx.z;
@@ -674,6 +679,7 @@ __global__ void __launch_bounds__(128)
                           const T *__restrict__ fx, const T *__restrict__ fy,
                           const uint2 *__restrict__ fp2, const double *__restrict__ t_x,
                           const double *__restrict__ t_y, Geometry g) {
+  chain_begin();
   const int c0 = blockIdx.x * 29;
   const int p0 = (blockIdx.y * blockDim.y + threadIdx.y) * RB;
   const int j = blockIdx.z;
@@ -770,9 +776,8 @@ cudaError_t launch_chain_adj(const double *lam, const double *mB, const MomentTa
                              const int64_t *ch_start, const int32_t *ch_len, int64_t nch,
                              int64_t ndrift, const Geometry &g, cudaStream_t st) {
   if (nch <= 0) return cudaSuccess;
-  chain_adj_kernel<<<(unsigned)((nch + 255) / 256), 256, 0, st>>>(
-      lam, mB, mt, ringb, tv, ch_cell, ch_start, ch_len, nch, ndrift, g);
-  return cudaGetLastError();
+  return chain_launch(chain_adj_kernel, dim3((unsigned)((nch + 255) / 256)), dim3(256), 0, st, lam,
+                      mB, mt, ringb, tv, ch_cell, ch_start, ch_len, nch, ndrift, g);
 }
 
 // SMs of the current device, looked up once per device
@@ -819,9 +824,8 @@ cudaError_t launch_drift_adj_gather(const double *lam, const double *mB, const M
   auto go = [&](auto kern, int R) {
     const dim3 grid((unsigned)((g.pc + 28) / 29), (unsigned)((g.nu + 3 + 4 * R - 1) / (4 * R)),
                     (unsigned)g.nj);
-    kern<<<grid, dim3(32, 4), 0, st>>>(lam, mB, mt, tv, Cb, ends, ent, ebase, fx, fy, fp2, t_x,
-                                       t_y, g);
-    return cudaGetLastError();
+    return chain_launch(kern, grid, dim3(32, 4), 0, st, lam, mB, mt, tv, Cb, ends, ent, ebase, fx,
+                        fy, fp2, t_x, t_y, g);
   };
   if (lane_waves(g, 32) >= 4.0) return go(drift_adj_lane_kernel<T, 32>, 32);
   return go(drift_adj_lane_kernel<T, 16>, 16);
@@ -841,8 +845,8 @@ cudaError_t launch_inv_geo(const uint32_t *ent, const int64_t *ebase, const uint
 cudaError_t launch_inv_perm(const uint32_t *ent, const int64_t *ebase, const double *lam,
                             const double *mB, const MomentTables &mt, const double *tv,
                             double *vperm, const Geometry &g, cudaStream_t st) {
-  inv_perm_kernel<<<slice_grid(g), 256, 0, st>>>(ent, ebase, lam, mB, mt, tv, vperm, g);
-  return cudaGetLastError();
+  return chain_launch(inv_perm_kernel, slice_grid(g), dim3(256), 0, st, ent, ebase, lam, mB, mt, tv,
+                      vperm, g);
 }
 
 cudaError_t launch_drift_adj_gather_perm(const double *vperm, const uint2 *geo, double *Cb,
@@ -853,8 +857,8 @@ cudaError_t launch_drift_adj_gather_perm(const double *vperm, const uint2 *geo, 
   auto go = [&](auto kern, int R) {
     const dim3 grid((unsigned)((g.pc + 32 * Q - 1) / (32 * Q)),
                     (unsigned)((g.nu + 3 + 4 * R - 1) / (4 * R)), (unsigned)g.nj);
-    kern<<<grid, dim3(32, 4), 0, st>>>(vperm, geo, Cb, ends, ebase, t_idx, t_x, t_y, g);
-    return cudaGetLastError();
+    return chain_launch(kern, grid, dim3(32, 4), 0, st, vperm, geo, Cb, ends, ebase, t_idx, t_x,
+                        t_y, g);
   };
   if (gather_waves(g, Q, 32) >= 4.0) return go(drift_adj_sweep_perm_kernel<32, Q>, 32);
   return go(drift_adj_sweep_perm_kernel<16, Q>, 16);
@@ -893,8 +897,8 @@ cudaError_t launch_ucol_adj(const T *f, double *Gb, double *A, double *B, double
 cudaError_t launch_shift_adj(const double *sbar, double *beta, unsigned int *count,
                              const MomentTables &mt, const Geometry &g, cudaStream_t st) {
   if (g.nr > 2048) return cudaErrorInvalidValue;
-  shift_adj_kernel<<<(g.nr + 31) / 32, 1024, 0, st>>>(sbar, beta, count, mt, g);
-  return cudaGetLastError();
+  return chain_launch(shift_adj_kernel, dim3((g.nr + 31) / 32), dim3(1024), 0, st, sbar, beta,
+                      count, mt, g);
 }
 
 cudaError_t launch_moment_adj(double *lam, const double *beta, const MomentTables &mt,

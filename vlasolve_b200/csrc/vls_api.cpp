@@ -1137,11 +1137,17 @@ static int drift_once(vls_handle *h, bool kick, const void *f_in = nullptr,
   const DirTables tr = dir_tables(h->tr, h->rp_r, h->q_r);
   const size_t gslot = (size_t)h->B * (h->co.nu + 2) * h->gp;
   const size_t cslot = (size_t)h->B * (h->co.nu + 3) * h->pc;
-  CK(h, cudaEventRecord(h->ev_fork, h->st));
-  for (int k = 0; k < h->NS; k++) CK(h, cudaStreamWaitEvent(h->bst[k], h->ev_fork, 0));
+  // several batch streams fork from the handle's stream and join it; a single
+  // one is the handle's stream itself, whose kernels then follow one another
+  // without an event between them (chained launches)
+  const bool fork = h->NS > 1;
+  if (fork) {
+    CK(h, cudaEventRecord(h->ev_fork, h->st));
+    for (int k = 0; k < h->NS; k++) CK(h, cudaStreamWaitEvent(h->bst[k], h->ev_fork, 0));
+  }
   for (int b = 0; b < h->nbatch; b++) {
     const int sl = b % h->NS;
-    cudaStream_t bs = h->bst[sl];
+    cudaStream_t bs = fork ? h->bst[sl] : h->st;
     Geometry g = geometry(h);
     g.j0 = b * h->B;
     g.nb = std::min(h->B, h->co.nj - g.j0);
@@ -1196,7 +1202,7 @@ static int drift_once(vls_handle *h, bool kick, const void *f_in = nullptr,
               },
               bs));
   }
-  for (int k = 0; k < h->NS; k++) {
+  for (int k = 0; fork && k < h->NS; k++) {
     CK(h, cudaEventRecord(h->ev_join[k], h->bst[k]));
     CK(h, cudaStreamWaitEvent(h->st, h->ev_join[k], 0));
   }

@@ -98,4 +98,37 @@ __device__ __forceinline__ void bulk_wait_read() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
 }
 
+// ------------------------------------------------------- chained launches
+// The kernels of a step follow one another in a stream.  A chained launch is
+// set up while the previous kernel runs and starts its blocks when that
+// kernel's blocks have left; chain_begin(), before a kernel's first access to
+// global memory, waits until the previous kernel is complete and its writes
+// are visible.  Every kernel launched this way does so first, so that what
+// lies before the previous kernel is complete as well.  About 3 us less
+// between two kernels: a step of 33 x 33 x 8 35 -> 25 us, 257 x 257 x 128
+// FP32 124 -> 114, 513 x 513 x 256 617 -> 604.
+//
+// No kernel lets the next one's blocks in earlier (launch_dependents): they
+// would run on SMs whose split of shared memory and L1 is still the previous
+// kernel's (201 x 201 x 200 FP64 177 -> 233 us a step, 513 x 513 x 256 604 ->
+// 666).
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline cudaError_t chain_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                                cudaStream_t st, A &&...args) {
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kern, P(args)...);
+}
+
 }  // namespace vls

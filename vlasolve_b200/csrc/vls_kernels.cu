@@ -705,6 +705,7 @@ __global__ void __launch_bounds__(DT_THREADS)
   const int jl = blockIdx.y, j = g.j0 + jl;  // batch-local / global slice
   const int nch = (g.nu + DW_CH - 1) / DW_CH;
   const int x0 = r0 - DW_XOFF;
+  chain_begin();
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     mbar_init(&bar[1], 1);
@@ -813,10 +814,8 @@ cudaError_t launch_drift_tma(const CUtensorMap *tmC, const T *C, T *f, const int
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((g.nr + 31) / 32, g.nb);
-  drift_tma_kernel<T><<<grid, DT_THREADS, smem, st>>>(*tmC, C, f, idx, fx, fy, fp2, ch_start,
-                                                       ch_len, ch_val, ndrift, mt, partial,
-                                                       err, spins, g);
-  return cudaGetLastError();
+  return chain_launch(drift_tma_kernel<T>, grid, dim3(DT_THREADS), smem, st, *tmC, C, f, idx, fx,
+                      fy, fp2, ch_start, ch_len, ch_val, ndrift, mt, partial, err, spins, g);
 }
 
 // ------------------------------------------------------------ strip drift
@@ -1130,6 +1129,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
     }
     mbar_fence_init();
   }
+  chain_begin();
   for (int u = tid; u < nt * DS_TRIP; u += 32 * (NW + 1)) bus[u] = __ldg(mt.bu32 + u);
   __syncthreads();
   const int nmine = (int)blockIdx.x < ntask ? (ntask - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -1380,9 +1380,9 @@ static cudaError_t drift_strip_go(const CUtensorMap *tmS, const float *C, float 
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return e;
   const int ntask = strip_blocks(g.nr) * g.nb;
-  drift_strip_kernel<NW, NB, MINB><<<std::min(ntask, nsm * MINB), 32 * (NW + 1), smem, st>>>(
-      *tmS, C, f, fp2, trip_kinds, mt, partial, err, spins, g);
-  return cudaGetLastError();
+  return chain_launch(drift_strip_kernel<NW, NB, MINB>, dim3(std::min(ntask, nsm * MINB)),
+                      dim3(32 * (NW + 1)), smem, st, *tmS, C, f, fp2, trip_kinds, mt, partial, err,
+                      spins, g);
 }
 
 cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C, float *f,
@@ -1420,6 +1420,7 @@ __global__ void __launch_bounds__(256)
                 const int32_t *__restrict__ chain_lo, int64_t ndrift,
                 const uint32_t *__restrict__ far_base, const uint32_t *__restrict__ far,
                 const uint2 *__restrict__ fp2, Geometry g) {
+  chain_begin();
   const int jl = blockIdx.y, j = g.j0 + jl;
   const T *Cj = C + (size_t)jl * (g.nu + 3) * g.pc;
   const size_t sb = (size_t)j * g.nu * g.nr;
@@ -1457,10 +1458,9 @@ cudaError_t launch_edge(const T *C, T *f, T *ch_val, const EdgeTables &t, int64_
                         const uint2 *fp2, int most, const Geometry &g, cudaStream_t st) {
   if (most <= 0) return cudaSuccess;
   auto go = [&](auto kern) {
-    kern<<<dim3((most + 255) / 256, g.nb), 256, 0, st>>>(
-        C, f, ch_val, t.ch_start, t.ch_len, t.ch_at, t.t_idx, t.t_x, t.t_y, t.chain_lo, ndrift,
-        t.far_base, t.far, fp2, g);
-    return cudaGetLastError();
+    return chain_launch(kern, dim3((most + 255) / 256, g.nb), dim3(256), 0, st, C, f, ch_val,
+                        t.ch_start, t.ch_len, t.ch_at, t.t_idx, t.t_x, t.t_y, t.chain_lo, ndrift,
+                        t.far_base, t.far, fp2, g);
   };
   if constexpr (sizeof(T) == 4)
     if (t.far_base) return go(edge_kernel<T, true>);
@@ -1472,6 +1472,7 @@ template <typename T>
 __global__ void __launch_bounds__(32 * DR_W)
     moment_kernel(const T *__restrict__ f, MomentTables mt,
                   double *__restrict__ partial, Geometry g) {
+  chain_begin();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int r = blockIdx.x * 32 + lane;
   const int j = blockIdx.y;
@@ -1494,8 +1495,7 @@ template <typename T>
 cudaError_t launch_moment(const T *f, const MomentTables &mt, double *partial,
                           const Geometry &g, cudaStream_t st) {
   dim3 grid((g.nr + 31) / 32, g.nj);
-  moment_kernel<T><<<grid, 32 * DR_W, 0, st>>>(f, mt, partial, g);
-  return cudaGetLastError();
+  return chain_launch(moment_kernel<T>, grid, dim3(32 * DR_W), 0, st, f, mt, partial, g);
 }
 
 // -------------------------------------------------------------- scan
@@ -1516,6 +1516,7 @@ __global__ void __launch_bounds__(SC_THREADS)
   __shared__ dd sh[SC_THREADS];
   __shared__ bool last;
   const int tid = threadIdx.x;
+  chain_begin();
   {
     const int lr = tid % SC_RB, jg = tid / SC_RB;  // 32 groups of J
     const int ngroups = SC_THREADS / SC_RB;
@@ -1601,9 +1602,8 @@ cudaError_t launch_scan(const double *partial, const MomentTables &mt,
                         const Geometry &g, cudaStream_t st) {
   if (g.nr > 2 * SC_THREADS) return cudaErrorInvalidValue;
   const unsigned blocks = (g.nr + SC_RB - 1) / SC_RB;
-  scan_kernel<<<blocks, SC_THREADS, 0, st>>>(partial, mt, T2, bins, Mr, shift, mtot,
-                                             count, status, g);
-  return cudaGetLastError();
+  return chain_launch(scan_kernel, dim3(blocks), dim3(SC_THREADS), 0, st, partial, mt, T2, bins, Mr,
+                      shift, mtot, count, status, g);
 }
 
 // ------------------------------------------------------------------ stats
@@ -1626,6 +1626,7 @@ __global__ void __launch_bounds__(ST_THREADS)
                  const double *__restrict__ dR, const double *__restrict__ dU,
                  const double *__restrict__ Ct1, double *__restrict__ part,
                  Geometry g) {
+  chain_begin();
   const int j = blockIdx.y;
   const int u0 = blockIdx.x * ST_U, u1 = min(u0 + ST_U, g.nu - 1);
   dd acc[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
@@ -1674,6 +1675,7 @@ __global__ void __launch_bounds__(ST_THREADS)
 // block q: quantity q of all block partials, in a fixed order
 __global__ void __launch_bounds__(ST_THREADS)
     stats_sum_kernel(const double *__restrict__ part, int nblk, double *__restrict__ out4) {
+  chain_begin();
   const int q = blockIdx.x;
   dd s{0, 0};
   for (int b = threadIdx.x; b < nblk; b += ST_THREADS) {
@@ -1698,11 +1700,11 @@ cudaError_t launch_stats(const T *f, const double *R, const double *U,
                          const double *Ct1, double *part, double *out4,
                          const Geometry &g, cudaStream_t st) {
   dim3 grid((g.nu - 1 + ST_U - 1) / ST_U, g.nj);
-  stats_kernel<T><<<grid, ST_THREADS, 0, st>>>(f, R, U, J, dR, dU, Ct1, part, g);
-  const cudaError_t e = cudaGetLastError();
+  const cudaError_t e = chain_launch(stats_kernel<T>, grid, dim3(ST_THREADS), 0, st, f, R, U, J,
+                                     dR, dU, Ct1, part, g);
   if (e != cudaSuccess) return e;
-  stats_sum_kernel<<<4, ST_THREADS, 0, st>>>(part, (int)stats_blocks(g.nu, g.nj), out4);
-  return cudaGetLastError();
+  return chain_launch(stats_sum_kernel, dim3(4), dim3(ST_THREADS), 0, st, part,
+                      (int)stats_blocks(g.nu, g.nj), out4);
 }
 
 // ------------------------------------------------------------ conversions

@@ -411,6 +411,7 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
   const bool colok = r < g.nr;
   const int jl = blockIdx.y, j = g.j0 + jl;
   const int kfirst = 1 + ro.s * L;
+  chain_begin();
   R v[L];
   {
     // unpredicated loads kept inside the slice (columns clamped to N_r - 1,
@@ -609,6 +610,7 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
   const int nrow = min(LN, rows - kr0);
   const T *Gs = G + ((size_t)jl * rows + kr0) * g.gp;
   bool landed = true;
+  chain_begin();
   if constexpr (BULK) {
     if (threadIdx.x == 0) {
       mbar_init(&bar, 1);
@@ -747,6 +749,7 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
       bulk_load(tile + p * P + OFF, Gs + (size_t)p * g.gp, gbytes, &bar[b]);
   };
   int issued = 0;  // groups whose loads thread 0 issued
+  chain_begin();
   if (threadIdx.x == 0) {
     for (int b = 0; b < RC_PIPE_TILES; ++b) mbar_init(&bar[b], 1);
     mbar_fence_init();
@@ -857,8 +860,7 @@ cudaError_t ucol_rc_go(const T *f, T *G, const double *shift, const Geometry &g,
   auto k = ucol_rc_kernel<T, R, KICK, CF>;
   cudaError_t e = rc_attr(k, smem);
   if (e != cudaSuccess) return e;
-  k<<<grid, nt, smem, st>>>(f, G, shift, g, tu);
-  return cudaGetLastError();
+  return chain_launch(k, grid, dim3(nt), smem, st, f, G, shift, g, tu);
 }
 
 // occupancy of the persistent r-solve per (device, kernel, shared memory,
@@ -943,8 +945,7 @@ cudaError_t prer_rc_go(const T *G, T *C, const Geometry &g, const RcDir<R> &tr,
         const int gps = (g.nu + 2 + CF::LN - 1) / CF::LN;
         const int ngroups = gps * g.nb;
         const int blocks = std::max(1, std::min(ngroups, nsm * per));
-        kp<<<blocks, nt, psmem, st>>>(G, C, g, tr, err, gps, ngroups);
-        return cudaGetLastError();
+        return chain_launch(kp, dim3(blocks), dim3(nt), psmem, st, G, C, g, tr, err, gps, ngroups);
       }
     }
   }
@@ -952,8 +953,7 @@ cudaError_t prer_rc_go(const T *G, T *C, const Geometry &g, const RcDir<R> &tr,
   auto k = prer_rc_kernel<T, R, CF>;
   cudaError_t e = rc_attr(k, smem);
   if (e != cudaSuccess) return e;
-  k<<<grid, nt, smem, st>>>(G, C, g, tr, err);
-  return cudaGetLastError();
+  return chain_launch(k, grid, dim3(nt), smem, st, G, C, g, tr, err);
 }
 
 // ----------------------------------------------------------- adjoint
@@ -1099,6 +1099,7 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
                        double *__restrict__ lam, double *__restrict__ sbar,
                        const double *__restrict__ shift, Geometry g,
                        const __grid_constant__ RcDir<double> t) {
+  chain_begin();
   constexpr int L = CF::L, LN = CF::LN;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int S = t.S, N = t.N;  // N == g.nu
@@ -1290,6 +1291,7 @@ template <class CF>
 __global__ void __launch_bounds__(CF::NT, CF::MINB)
     prer_adj_rc_kernel(const double *__restrict__ Cb, double *__restrict__ Gb, Geometry g,
                        const __grid_constant__ RcDir<double> t) {
+  chain_begin();
   constexpr int L = CF::L, LN = CF::LN;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const int S = t.S, N = t.N;  // N == g.nr
@@ -1495,8 +1497,7 @@ static cudaError_t ucol_adj_go(const T *f, const double *Gb, double *lam, double
   cudaError_t e = rc_attr(k, smem);
   if (e != cudaSuccess) return e;
   const dim3 grid((g.nr + CF::LN - 1) / CF::LN, g.nj);
-  k<<<grid, nt, smem, st>>>(f, Gb, lam, sbar, shift, g, tu);
-  return cudaGetLastError();
+  return chain_launch(k, grid, dim3(nt), smem, st, f, Gb, lam, sbar, shift, g, tu);
 }
 
 template <typename T>
@@ -1518,8 +1519,7 @@ static cudaError_t prer_adj_go(const double *Cb, double *Gb, const Geometry &g,
   cudaError_t e = rc_attr(k, smem);
   if (e != cudaSuccess) return e;
   const dim3 grid((g.nu + 2 + CF::LN - 1) / CF::LN, g.nj);
-  k<<<grid, nt, smem, st>>>(Cb, Gb, g, tr);
-  return cudaGetLastError();
+  return chain_launch(k, grid, dim3(nt), smem, st, Cb, Gb, g, tr);
 }
 
 cudaError_t launch_prer_adj_rc(const double *Cb, double *Gb, const Geometry &g,
