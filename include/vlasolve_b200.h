@@ -123,7 +123,7 @@ int vls_create(const vls_grid_desc *grid, const vls_solver_desc *solver,
      drift             VLS_DRIFT_AUTO: FP32 storage stages whole coefficient
                        strips (two strip buffers per block where they fit,
                        else one), FP64 storage and strips too tall for one
-                       block take staged 64 x 40 windows; VLS_DRIFT_WINDOW /
+                       block take staged windows; VLS_DRIFT_WINDOW /
                        _STRIP2 / _STRIP1 ask for one of those (a strip that
                        does not fit, or FP64, falls back to windows).
      slices_per_batch  J slices per batch of the prefilter and drift scratch

@@ -43,6 +43,7 @@ struct vls_handle {
   // the strip drift's tables for these footpoints: trip kinds, and the
   // far-tap cells (their number per slice on the host)
   uint8_t *trip_kinds = nullptr;
+  int16_t *win_rows = nullptr;  // window rows of the windowed drift
   uint32_t *far_base = nullptr, *far_count = nullptr, *far = nullptr;
   size_t far_cap = 0;
   std::vector<uint32_t> far_base_h;
@@ -307,12 +308,20 @@ static uint2 encode_packed(const Coords &c, int32_t code, double rF, double uF) 
   return w;
 }
 
-// The footpoint tables are new: the strip drift's tables follow them.
+// The footpoint tables are new: the drift kernels' tables follow them.
 static int footpoints_changed(vls_handle *h) {
   h->fp_gen++;
   const Coords &c = h->co;
   h->far_base_h.assign((size_t)c.nj + 1, 0);
-  if (h->drift_kind == DRIFT_WINDOW) return VLS_OK;
+  if (h->drift_kind == DRIFT_WINDOW) {
+    if (!h->win_rows)
+      TRY(dalloc(h, &h->win_rows, sizeof(int16_t) * window_rows_count(c.nr, c.nu, c.nj)));
+    CK(h, h->esize == 8 ? launch_window_rows<double>(h->idx, h->fp2, h->win_rows, c.nr, c.nu, c.nj,
+                                                     h->st)
+                        : launch_window_rows<float>(h->idx, h->fp2, h->win_rows, c.nr, c.nu, c.nj,
+                                                    h->st));
+    return VLS_OK;
+  }
   if (!h->trip_kinds) {
     TRY(dalloc(h, &h->trip_kinds, trip_kinds_bytes(c.nr, c.nu, c.nj)));
     TRY(dalloc(h, &h->far_count, sizeof(uint32_t) * c.nj));
@@ -498,8 +507,8 @@ static int setup_chain_device(vls_handle *h) {
   return VLS_OK;
 }
 
-// 3D tiled tensor maps of C ([N_J][N_u+3][pc], element T): boxes of 64
-// columns x 40 rows x 1 slice for the drift windows, 48 columns x
+// 3D tiled tensor maps of C ([N_J][N_u+3][pc], element T): boxes of DW_COLS
+// columns x DW_ROWS rows x 1 slice for the drift windows, 48 columns x
 // drift_strip_box_rows x 1 slice for the strips.  The encoder is the driver's cuTensorMapEncodeTiled,
 // reached through the runtime (no libcuda link).  Returns false when it is
 // unavailable or refuses a map (vls_create then fails: every drift kernel
@@ -521,7 +530,7 @@ static bool make_tensor_map(vls_handle *h) {
                                 (cuuint64_t)h->B};
     const cuuint64_t strides[2] = {(cuuint64_t)h->pc * es,
                                    (cuuint64_t)h->pc * es * (cuuint64_t)(h->co.nu + 3)};
-    const cuuint32_t box[3] = {64, 40, 1};
+    const cuuint32_t box[3] = {DW_COLS, DW_ROWS, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     void *base = (char *)h->C + s * slot * es;
     const CUresult r = enc(&h->tmC[s],
@@ -1196,8 +1205,8 @@ static int drift_once(vls_handle *h, bool kick, const void *f_in = nullptr,
                                               h->flag + 1, h->drift_spins, g, bs);
                 }
                 return launch_drift_tma<T>(&h->tmC[sl], C, fout, h->idx, (const T *)h->fx,
-                                           (const T *)h->fy, h->fp2, h->ch_start, h->ch_len,
-                                           (const T *)h->ch_val, h->ndrift, moment_tables(h),
+                                           (const T *)h->fy, h->fp2, h->win_rows, h->ch_start,
+                                           h->ch_len, (const T *)h->ch_val, h->ndrift, moment_tables(h),
                                            h->partial, h->flag + 1, h->drift_spins, g, bs);
               },
               bs));

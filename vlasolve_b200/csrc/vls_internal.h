@@ -96,18 +96,29 @@ cudaError_t launch_prer(const T *G, T *C, const Geometry &g, const DirTables &tr
                         cudaStream_t st);
 // drift kernels (the values of the public VLS_DRIFT_* layout choices)
 constexpr int DRIFT_AUTO = 0, DRIFT_WINDOW = 1, DRIFT_STRIP2 = 2, DRIFT_STRIP1 = 3;
+// the windowed drift's staged windows, columns x rows of coefficients (the
+// box of its tensor map).  FP64 drift of 513 x 513 x 128 / 201 x 201 x 200:
+// 48 x 48 0.305 / 0.0946 ms, 48 x 40 0.308 / 0.0958, 48 x 56 0.311 / 0.0942,
+// 64 x 32 0.315 / 0.0977, 64 x 40 0.313 / 0.0980, 64 x 48 0.410 / 0.110
+constexpr int DW_COLS = 48, DW_ROWS = 48;
 // footpoints: FP64 handles use idx/fx/fy, FP32 handles the packed fp2 table.
 // Drift with the coefficient windows staged by TMA (tmC: 3D map of C, box
-// 64 columns x 40 rows x 1 slice); err receives bit 0 when a wait for a
+// DW_COLS columns x DW_ROWS rows x 1 slice); err receives bit 0 when a wait for a
 // window ran out after `spins` polls (the cells then read C in global
 // memory), bit 1 when a copy had still not landed at the block's end
 template <typename T>
 cudaError_t launch_drift_tma(const CUtensorMap *tmC, const T *C, T *f, const int32_t *idx,
-                             const T *fx, const T *fy, const uint2 *fp2,
+                             const T *fx, const T *fy, const uint2 *fp2, const int16_t *win_rows,
                              const int64_t *ch_start, const int32_t *ch_len,
                              const T *ch_val, int64_t ndrift, const MomentTables &mt,
                              double *partial, unsigned int *err, uint32_t spins,
                              const Geometry &g, cudaStream_t st);
+// win_rows: the first row of each (slice, strip, chunk)'s window, from the
+// footpoints of all slices
+size_t window_rows_count(int nr, int nu, int nj);
+template <typename T>
+cudaError_t launch_window_rows(const int32_t *idx, const uint2 *fp2, int16_t *rows, int nr, int nu,
+                               int nj, cudaStream_t st);
 // drift from whole coefficient strips staged by TMA (tmS: 3D map of C, box 48
 // columns x drift_strip_box_rows x 1 slice).  drift_strip_width returns the
 // strip kind (DRIFT_STRIP2 / DRIFT_STRIP1) the grid takes, or DRIFT_WINDOW

@@ -601,7 +601,16 @@ __device__ __forceinline__ float2 frac21x2(uint2 w) {
 // are read from shared memory; footpoints outside it (far displacements) read
 // the coefficients from global memory.  Every mbarrier wait is bounded: on
 // timeout the block records an error flag and falls back to global reads.
-constexpr int DW_COLS = 64, DW_ROWS = 40, DW_CH = 16, DW_XOFF = 16, DW_YOFF = 12;
+//
+// Footpoints are fixed for the run, so each window's first row is chosen once
+// per chunk (window_rows_kernel): the one that holds most of the chunk's tap
+// blocks, which drift together by up to hundreds of rows at small radii (4.7 %
+// of the in-box cells of the 513 x 513 Hernquist grid lie outside it, 10.8 %
+// outside windows that start 12 rows above their chunk).  Chunks with every
+// cell outside the box (20 % of them) store zeros, stage nothing and read no
+// footpoints.  FP64 drift 0.379 -> 0.305 ms on 513 x 513 x 128 Hernquist,
+// 0.106 -> 0.095 on 201 x 201 x 200 UDF, the narrower windows included.
+constexpr int DW_CH = 16, DW_XOFF = (DW_COLS - 32) / 2;
 constexpr int DT_THREADS = 256;  // 8 warps x 32 columns; 2 rows per warp per chunk
 template <typename T>
 struct Cell {
@@ -685,13 +694,88 @@ __device__ __forceinline__ float eval_window<float>(const float *p, float x, flo
   return gather_f32x2([&](int a, int b) { return p[a * DW_COLS + b]; }, x, y);
 }
 
+constexpr int DW_MAX_CH = 2048 / DW_CH;   // chunks of the tallest slice
+constexpr int16_t DW_EMPTY = INT16_MIN;  // a chunk with nothing to gather or read
+
+// first window row of each (slice, strip, chunk): one warp each
+template <typename T>
+__global__ void __launch_bounds__(128)
+    window_rows_kernel(const int32_t *__restrict__ idx, const uint2 *__restrict__ fp2,
+                       int16_t *__restrict__ rows, int nr, int nu, int nj) {
+  __shared__ uint16_t hist[4][2048];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int ns = (nr + 31) / 32, nch = (nu + DW_CH - 1) / DW_CH;
+  const size_t k = (size_t)blockIdx.x * 4 + w;
+  if (k >= (size_t)nj * ns * nch) return;
+  const int c = (int)(k % nch), s = (int)(k / nch % ns);
+  const size_t j = k / ((size_t)nch * ns);
+  uint16_t *h = hist[w];
+  for (int y = lane; y < 2048; y += 32) h[y] = 0;
+  __syncwarp();
+  const int r = 32 * s + lane, x0 = 32 * s - DW_XOFF;
+  bool some = false;
+  for (int u = c * DW_CH; u < min((c + 1) * DW_CH, nu); ++u) {
+    int y = -1;
+    if (r < nr) {
+      const size_t cell = (j * nu + u) * nr + r;
+      int rI;
+      if constexpr (sizeof(T) == 4) {
+        const uint2 q = __ldg(fp2 + cell);
+        some = some || q.x != FP_OUT;
+        rI = (int)(q.x >> FP_FBITS);
+        y = q.x < FP_CHAIN ? (int)(q.y >> FP_FBITS) : -1;
+      } else {
+        const int code = __ldg(idx + cell);
+        some = some || code != -1;
+        rI = code & 0xffff;
+        y = code >= 0 ? code >> 16 : -1;
+      }
+      if (rI - x0 < 0 || rI - x0 > DW_COLS - 4) y = -1;
+    }
+    // lanes with the same row add once
+    const unsigned same = __match_any_sync(0xffffffffu, y);
+    if (y >= 0 && lane == __ffs(same) - 1) h[y] += (uint16_t)__popc(same);
+    __syncwarp();
+  }
+  // the start whose DW_ROWS - 3 tap rows hold most cells, the first of equals
+  int best = -1, by = 0;
+  for (int y = lane; y < nu; y += 32) {
+    int n = 0;
+    for (int q = y; q < min(y + DW_ROWS - 3, nu); ++q) n += h[q];
+    if (n > best) {
+      best = n;
+      by = y;
+    }
+  }
+  for (int d = 16; d > 0; d >>= 1) {
+    const int n = __shfl_xor_sync(0xffffffffu, best, d), y = __shfl_xor_sync(0xffffffffu, by, d);
+    if (n > best || (n == best && y < by)) {
+      best = n;
+      by = y;
+    }
+  }
+  some = __any_sync(0xffffffffu, some);
+  if (lane == 0) rows[k] = some ? (int16_t)by : DW_EMPTY;
+}
+
+size_t window_rows_count(int nr, int nu, int nj) {
+  return (size_t)nj * ((nr + 31) / 32) * ((nu + DW_CH - 1) / DW_CH);
+}
+template <typename T>
+cudaError_t launch_window_rows(const int32_t *idx, const uint2 *fp2, int16_t *rows, int nr, int nu,
+                               int nj, cudaStream_t st) {
+  window_rows_kernel<T><<<(unsigned)((window_rows_count(nr, nu, nj) + 3) / 4), 128, 0, st>>>(
+      idx, fp2, rows, nr, nu, nj);
+  return cudaGetLastError();
+}
+
 template <typename T>
 __global__ void __launch_bounds__(DT_THREADS)
     drift_tma_kernel(const __grid_constant__ CUtensorMap tmC, const T *__restrict__ C,
                      T *__restrict__ f,
                      const int32_t *__restrict__ idx, const T *__restrict__ fx,
                      const T *__restrict__ fy, const uint2 *__restrict__ fp2,
-                     const int64_t *__restrict__ ch_start, const int32_t *__restrict__ ch_len,
+                     const int16_t *__restrict__ win_rows, const int64_t *__restrict__ ch_start, const int32_t *__restrict__ ch_len,
                      const T *__restrict__ ch_val, int64_t ndrift, MomentTables mt,
                      double *__restrict__ partial, unsigned int *err, uint32_t spins,
                      Geometry g) {
@@ -705,51 +789,69 @@ __global__ void __launch_bounds__(DT_THREADS)
   const int jl = blockIdx.y, j = g.j0 + jl;  // batch-local / global slice
   const int nch = (g.nu + DW_CH - 1) / DW_CH;
   const int x0 = r0 - DW_XOFF;
-  chain_begin();
-  if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_fence_init();
-    for (int c = 0; c < 2 && c < nch; ++c) {
-      mbar_expect_tx(&bar[c], BYTES);
-      tma_load_3d(win + c * DW_COLS * DW_ROWS, &tmC, x0, c * DW_CH - DW_YOFF, jl, &bar[c]);
-    }
-  }
-  __syncthreads();
-  const T *Cj = C + (size_t)jl * (g.nu + 3) * g.pc;
+  // the chunks' window rows, and the list of those that are not empty
+  __shared__ int16_t wy[DW_MAX_CH];
+  __shared__ uint8_t list[DW_MAX_CH];
+  __shared__ int nlist;
   const size_t row0 = (size_t)j * g.nu * g.nr + r;
   const bool col_ok = r < g.nr;
   RawCell<T> nxt[2];
+  auto words_of = [&](int c) {
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const int u = w + 8 * q;
-    nxt[q] = load_raw(idx, fx, fy, fp2, row0 + (size_t)(u < g.nu && col_ok ? u : 0) * g.nr);
-  }
-  double acc = 0.0;
-  // copy bookkeeping (meaningful in thread 0, which issues every copy): the
-  // chunk last sent to each buffer and whether its completion was observed
-  int last0 = 0, last1 = 1;                   // chunk last sent to buffer 0 / 1
-  unsigned pending = 1u | (nch > 1 ? 2u : 0u);  // bit b: buffer b's copy not yet seen
-  bool issuing = true;
-  for (int c = 0; c < nch; ++c) {
-    const RawCell<T> cur[2] = {nxt[0], nxt[1]};
-    if (c + 1 < nch) {
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int u = (c + 1) * DW_CH + w + 8 * q;
-        nxt[q] = load_raw(idx, fx, fy, fp2, row0 + (size_t)(u < g.nu && col_ok ? u : 0) * g.nr);
+    for (int q = 0; q < 2; ++q) {
+      const int u = c * DW_CH + w + 8 * q;
+      nxt[q] = load_raw(idx, fx, fy, fp2, row0 + (size_t)(u < g.nu && col_ok ? u : 0) * g.nr);
+    }
+  };
+  chain_begin();
+  words_of(0);  // the first chunk's, unless it turns out to be empty
+  if (w == 0) {
+    const int16_t *src = win_rows + ((size_t)j * gridDim.x + blockIdx.x) * nch;
+    int n = 0;
+    for (int c0 = 0; c0 < nch; c0 += 32) {
+      const int c = c0 + lane;
+      const int16_t y = c < nch ? __ldg(src + c) : DW_EMPTY;
+      const unsigned m = __ballot_sync(0xffffffffu, y != DW_EMPTY);
+      if (c < nch) wy[c] = y;
+      if (y != DW_EMPTY) list[n + __popc(m & ((1u << lane) - 1u))] = (uint8_t)c;
+      n += __popc(m);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      nlist = n;
+      mbar_init(&bar[0], 1);
+      mbar_init(&bar[1], 1);
+      mbar_fence_init();
+      for (int k = 0; k < 2 && k < n; ++k) {
+        mbar_expect_tx(&bar[k], BYTES);
+        tma_load_3d(win + k * DW_COLS * DW_ROWS, &tmC, x0, wy[list[k]], jl, &bar[k]);
       }
     }
-    const int b = c & 1;
+  }
+  __syncthreads();
+  const int nl = nlist;
+  const T *Cj = C + (size_t)jl * (g.nu + 3) * g.pc;
+  if (nl > 0 && list[0] != 0) words_of(list[0]);
+  double acc = 0.0;
+  // copy bookkeeping (meaningful in thread 0, which issues every copy): the
+  // list entry last sent to each buffer and whether its completion was observed
+  int last0 = 0, last1 = 1;
+  unsigned pending = (nl > 0 ? 1u : 0u) | (nl > 1 ? 2u : 0u);  // bit b: buffer b's copy not yet seen
+  bool issuing = true;
+  for (int k = 0; k < nl; ++k) {
+    const int c = list[k];
+    const RawCell<T> cur[2] = {nxt[0], nxt[1]};
+    if (k + 1 < nl) words_of(list[k + 1]);
+    const int b = k & 1;
     // after one failed wait this thread waits no more (it reads C globally)
-    const bool have = issuing && mbar_wait_bounded(&bar[b], (uint32_t)((c >> 1) & 1), spins);
+    const bool have = issuing && mbar_wait_bounded(&bar[b], (uint32_t)((k >> 1) & 1), spins);
     if (have) pending &= ~(1u << b);
     if (!have && issuing) {
       issuing = false;  // never stack a second copy onto an unfinished one
       atomicOr(err, 1u);
     }
     const T *wb = win + b * DW_COLS * DW_ROWS;
-    const int y0 = c * DW_CH - DW_YOFF;
+    const int y0 = wy[c];
     T part = T(0);
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
@@ -773,13 +875,21 @@ __global__ void __launch_bounds__(DT_THREADS)
     }
     acc += (double)part;
     __syncthreads();  // every warp is done with window b
-    if (tid == 0 && issuing && c + 2 < nch) {
+    if (tid == 0 && issuing && k + 2 < nl) {
       fence_proxy_async();
       mbar_expect_tx(&bar[b], BYTES);
-      tma_load_3d(win + b * DW_COLS * DW_ROWS, &tmC, x0, (c + 2) * DW_CH - DW_YOFF, jl,
-                  &bar[b]);
-      if (b) last1 = c + 2; else last0 = c + 2;
+      tma_load_3d(win + b * DW_COLS * DW_ROWS, &tmC, x0, wy[list[k + 2]], jl, &bar[b]);
+      if (b) last1 = k + 2; else last0 = k + 2;
       pending |= 1u << b;
+    }
+  }
+  // the empty chunks
+  for (int c = 0; c < nch; ++c) {
+    if (wy[c] != DW_EMPTY) continue;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int u = c * DW_CH + w + 8 * q;
+      if (u < g.nu && col_ok) f[row0 + (size_t)u * g.nr] = T(0);
     }
   }
   // a copy whose wait timed out may still be in flight: wait for it (bounded)
@@ -787,7 +897,7 @@ __global__ void __launch_bounds__(DT_THREADS)
   if (tid == 0) {
     for (int b = 0; b < 2; ++b) {
       const int lb = b ? last1 : last0;
-      if (((pending >> b) & 1u) && lb < nch &&
+      if (((pending >> b) & 1u) && lb < nl &&
           !mbar_wait_bounded(&bar[b], (uint32_t)((lb >> 1) & 1)))
         atomicOr(err, 2u);
     }
@@ -804,7 +914,7 @@ __global__ void __launch_bounds__(DT_THREADS)
 
 template <typename T>
 cudaError_t launch_drift_tma(const CUtensorMap *tmC, const T *C, T *f, const int32_t *idx,
-                             const T *fx, const T *fy, const uint2 *fp2,
+                             const T *fx, const T *fy, const uint2 *fp2, const int16_t *win_rows,
                              const int64_t *ch_start, const int32_t *ch_len,
                              const T *ch_val, int64_t ndrift, const MomentTables &mt,
                              double *partial, unsigned int *err, uint32_t spins,
@@ -815,7 +925,7 @@ cudaError_t launch_drift_tma(const CUtensorMap *tmC, const T *C, T *f, const int
   if (e != cudaSuccess) return e;
   dim3 grid((g.nr + 31) / 32, g.nb);
   return chain_launch(drift_tma_kernel<T>, grid, dim3(DT_THREADS), smem, st, *tmC, C, f, idx, fx,
-                      fy, fp2, ch_start, ch_len, ch_val, ndrift, mt, partial, err, spins, g);
+                      fy, fp2, win_rows, ch_start, ch_len, ch_val, ndrift, mt, partial, err, spins, g);
 }
 
 // ------------------------------------------------------------ strip drift
@@ -1762,9 +1872,11 @@ cudaError_t launch_nonfinite(const T *f, size_t n, unsigned int *flag,
   template int drift_strip_width<T>(int, int);                                  \
   template cudaError_t launch_drift_tma<T>(                                     \
       const CUtensorMap *, const T *, T *, const int32_t *, const T *, const T *, \
-      const uint2 *, const int64_t *, const int32_t *, const T *, int64_t,        \
-      const MomentTables &, double *, unsigned int *, uint32_t, const Geometry &, \
-      cudaStream_t);                                                            \
+      const uint2 *, const int16_t *, const int64_t *, const int32_t *, const T *, \
+      int64_t, const MomentTables &, double *, unsigned int *, uint32_t,         \
+      const Geometry &, cudaStream_t);                                          \
+  template cudaError_t launch_window_rows<T>(const int32_t *, const uint2 *, int16_t *, int, \
+                                             int, int, cudaStream_t);           \
   template cudaError_t launch_edge<T>(const T *, T *, T *, const EdgeTables &, int64_t, \
                                       const uint2 *, int, const Geometry &, cudaStream_t); \
   template cudaError_t launch_moment<T>(const T *, const MomentTables &,        \
