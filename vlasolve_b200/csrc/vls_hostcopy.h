@@ -40,8 +40,9 @@ class ChunkPool {
     void *p[2] = {nullptr, nullptr};
   };
   static ChunkPool &get() {
-    static ChunkPool pool;
-    return pool;
+    // never destroyed: objects with static storage may still copy at exit
+    static ChunkPool *pool = new ChunkPool;
+    return *pool;
   }
   void user(int d) {
     std::lock_guard<std::mutex> lk(m_);

@@ -1209,7 +1209,7 @@ int drift_strip_box_rows(int nu) { return strip_smem(nu, 1, 1).rows; }
 // for a strip.  A block per strip with 16 x 2 warps per SM, every cell with
 // its 16 taps and the rare cells gathered in place, took 0.309 ms on the 513 x
 // 513 x 256 Hernquist case, 0.372 on 1025 x 1025 x 64 PLDF and 0.057 on 257 x
-// 257 x 128 Plummer (116 instructions per cell); this form 0.258, 0.305 and
+// 257 x 128 Plummer (116 instructions per cell); this form 0.261, 0.306 and
 // 0.049, and edge_kernel 0.012, 0.018 and 0.000 more than the tails alone.
 //
 // Waits are bounded.  A consumer whose wait for a strip ran out (`spins`
