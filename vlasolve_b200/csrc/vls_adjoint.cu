@@ -202,7 +202,7 @@ __global__ void ucol_adj_kernel(const T *__restrict__ f, double *__restrict__ Gb
 // exclusive scan over the radii, compensated as the forward's enclosed-mass
 // scan, and writes the moment term over the scratch.  The summation order is
 // fixed.
-__global__ void __launch_bounds__(1024) shift_adj_kernel(const double *__restrict__ sbar,
+__global__ void __launch_bounds__(1024) shift_adj_kernel(const double *sbar,
                                                          double *beta, unsigned int *count,
                                                          MomentTables mt, Geometry g) {
   chain_begin();
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(1024) shift_adj_kernel(const double *__restric
     double s = 0.0;
     if (r < g.nr) {
 #pragma unroll 8
-      for (int j = w; j < g.nj; j += 32) s += __ldg(sbar + (size_t)j * g.nr + r);
+      for (int j = w; j < g.nj; j += 32) s += sbar[(size_t)j * g.nr + r];
     }
     part[w][lane] = s;
     __syncthreads();
@@ -436,7 +436,7 @@ __global__ void inv_sort_kernel(const uint32_t *__restrict__ ends, uint32_t *__r
 // value this step's tails wrote) moves to tv for the gather and is cleared.
 // In the forward the tails write before the drift reads, so with L = 1 the
 // front add comes first here.
-__global__ void chain_adj_kernel(const double *__restrict__ lam, const double *__restrict__ mB,
+__global__ void chain_adj_kernel(const double *lam, const double *mB,
                                  MomentTables mt, double *__restrict__ ringb,
                                  double *__restrict__ tv, const int64_t *__restrict__ ch_cell,
                                  const int64_t *__restrict__ ch_start,
@@ -499,9 +499,9 @@ __global__ void inv_geo_kernel(const uint32_t *__restrict__ ent,
 
 // values of this transposed step in entry order
 __global__ void inv_perm_kernel(const uint32_t *__restrict__ ent,
-                                const int64_t *__restrict__ ebase, const double *__restrict__ lam,
-                                const double *__restrict__ mB, MomentTables mt,
-                                const double *__restrict__ tv, double *__restrict__ vperm,
+                                const int64_t *__restrict__ ebase, const double *lam,
+                                const double *mB, MomentTables mt, const double *tv,
+                                double *__restrict__ vperm,
                                 Geometry g) {
   chain_begin();
   const int j = blockIdx.y;
@@ -582,7 +582,7 @@ __device__ __forceinline__ void sweep_nodes(const Entry &entry, double *__restri
 
 template <int RB, int Q>
 __global__ void __launch_bounds__(128)
-    drift_adj_sweep_perm_kernel(const double *__restrict__ vperm, const uint2 *__restrict__ geo,
+    drift_adj_sweep_perm_kernel(const double *vperm, const uint2 *__restrict__ geo,
                                 double *__restrict__ Cb, const uint32_t *__restrict__ ends,
                                 const int64_t *__restrict__ ebase,
                                 const int32_t *__restrict__ t_idx,
@@ -672,8 +672,8 @@ __device__ __forceinline__ void lane_nodes(const Entry &entry, double *__restric
 
 template <typename T, int RB>
 __global__ void __launch_bounds__(128)
-    drift_adj_lane_kernel(const double *__restrict__ lam, const double *__restrict__ mB,
-                          MomentTables mt, const double *__restrict__ tv,
+    drift_adj_lane_kernel(const double *lam, const double *mB,
+                          MomentTables mt, const double *tv,
                           double *__restrict__ Cb, const uint32_t *__restrict__ ends,
                           const uint32_t *__restrict__ ent, const int64_t *__restrict__ ebase,
                           const T *__restrict__ fx, const T *__restrict__ fy,

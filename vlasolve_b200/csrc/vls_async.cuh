@@ -108,6 +108,14 @@ __device__ __forceinline__ void bulk_wait_read() {
 // between two kernels: a step of 33 x 33 x 8 35 -> 25 us, 257 x 257 x 128
 // FP32 124 -> 114, 513 x 513 x 256 617 -> 604.
 //
+// What the previous kernels of the stream wrote (f, G, C, shift, partial, the
+// chains' rings, the adjoint's fields) is read by plain loads through pointers
+// that are not __restrict__: the read-only path (__ldg, or what the compiler
+// makes of a const __restrict__ argument) is for data that stays constant over
+// the kernel's whole life, which here begins before those writes are visible,
+// and such a load may be scheduled above the wait.  Tables that no kernel of a
+// step writes may keep it.
+//
 // No kernel lets the next one's blocks in earlier (launch_dependents): they
 // would run on SMs whose split of shared memory and L1 is still the previous
 // kernel's (201 x 201 x 200 FP64 177 -> 233 us a step, 513 x 513 x 256 604 ->

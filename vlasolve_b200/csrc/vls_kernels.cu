@@ -493,22 +493,17 @@ cudaError_t launch_prer(const T *G, T *C, const Geometry &g, const DirTables &tr
 // localSpline::evaluateC(int,double,int,double), localSpline.hxx:381-398:
 // taps at padded columns rI..rI+3 and rows uI..uI+3 (FP64 form).
 template <typename T>
-__device__ __forceinline__ T eval2d(const T *__restrict__ Cj, int pc, int rI,
-                                    T x, int uI, T y) {
+__device__ __forceinline__ T eval2d(const T *Cj, int pc, int rI, T x, int uI, T y) {
   const T b2xI = bv2<T>(T(1) - x), b1xI = bv1<T>(T(1) - x);
   const T b1x = bv1<T>(x), b2x = bv2<T>(x);
   const T *p = Cj + (size_t)uI * pc + rI;
-  const T s0 = __ldg(p) * b2xI + __ldg(p + 1) * b1xI + __ldg(p + 2) * b1x +
-               __ldg(p + 3) * b2x;
+  const T s0 = p[0] * b2xI + p[1] * b1xI + p[2] * b1x + p[3] * b2x;
   p += pc;
-  const T s1 = __ldg(p) * b2xI + __ldg(p + 1) * b1xI + __ldg(p + 2) * b1x +
-               __ldg(p + 3) * b2x;
+  const T s1 = p[0] * b2xI + p[1] * b1xI + p[2] * b1x + p[3] * b2x;
   p += pc;
-  const T s2 = __ldg(p) * b2xI + __ldg(p + 1) * b1xI + __ldg(p + 2) * b1x +
-               __ldg(p + 3) * b2x;
+  const T s2 = p[0] * b2xI + p[1] * b1xI + p[2] * b1x + p[3] * b2x;
   p += pc;
-  const T s3 = __ldg(p) * b2xI + __ldg(p + 1) * b1xI + __ldg(p + 2) * b1x +
-               __ldg(p + 3) * b2x;
+  const T s3 = p[0] * b2xI + p[1] * b1xI + p[2] * b1x + p[3] * b2x;
   return over36<T>(bv2<T>(T(1) - y) * s0 + bv1<T>(T(1) - y) * s1 +
                            bv1<T>(y) * s2 + bv2<T>(y) * s3);
 }
@@ -558,16 +553,16 @@ __device__ __forceinline__ float gather_f32x2(const Ld &ld, float x, float y) {
 }
 
 // from C in global memory (row pitch pc), taps from Cj + off
-__device__ __forceinline__ float eval2d_f32x2(const float *__restrict__ Cj, int pc,
-                                              int off, float x, float y) {
+__device__ __forceinline__ float eval2d_f32x2(const float *Cj, int pc, int off, float x,
+                                              float y) {
   const float *p = Cj + off;
-  return gather_f32x2([&](int a, int b) { return __ldg(p + a * pc + b); }, x, y);
+  return gather_f32x2([&](int a, int b) { return p[a * pc + b]; }, x, y);
 }
 
 // FP32 storage: every gather in the difference form
 template <>
-__device__ __forceinline__ float eval2d<float>(const float *__restrict__ Cj, int pc, int rI,
-                                               float x, int uI, float y) {
+__device__ __forceinline__ float eval2d<float>(const float *Cj, int pc, int rI, float x, int uI,
+                                               float y) {
   return eval2d_f32x2(Cj, pc, uI * pc + rI, x, y);
 }
 
@@ -771,12 +766,13 @@ cudaError_t launch_window_rows(const int32_t *idx, const uint2 *fp2, int16_t *ro
 
 template <typename T>
 __global__ void __launch_bounds__(DT_THREADS)
-    drift_tma_kernel(const __grid_constant__ CUtensorMap tmC, const T *__restrict__ C,
+    drift_tma_kernel(const __grid_constant__ CUtensorMap tmC, const T *C,
                      T *__restrict__ f,
                      const int32_t *__restrict__ idx, const T *__restrict__ fx,
                      const T *__restrict__ fy, const uint2 *__restrict__ fp2,
-                     const int16_t *__restrict__ win_rows, const int64_t *__restrict__ ch_start, const int32_t *__restrict__ ch_len,
-                     const T *__restrict__ ch_val, int64_t ndrift, MomentTables mt,
+                     const int16_t *__restrict__ win_rows,
+                     const int64_t *__restrict__ ch_start, const int32_t *__restrict__ ch_len,
+                     const T *ch_val, int64_t ndrift, MomentTables mt,
                      double *__restrict__ partial, unsigned int *err, uint32_t spins,
                      Geometry g) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -1218,7 +1214,7 @@ int drift_strip_box_rows(int nu) { return strip_smem(nu, 1, 1).rows; }
 // before the block ends, whatever the consumers did.
 template <int NW, int NB, int MINB>
 __global__ void __launch_bounds__(32 * (NW + 1), MINB)
-    drift_strip_kernel(const __grid_constant__ CUtensorMap tmS, const float *__restrict__ C,
+    drift_strip_kernel(const __grid_constant__ CUtensorMap tmS, const float *C,
                        float *f, const uint2 *__restrict__ fp2,
                        const uint8_t *__restrict__ trip_kinds, MomentTables mt,
                        double *__restrict__ partial, unsigned int *err, uint32_t spins,
@@ -1527,7 +1523,7 @@ cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C,
 // less here, nothing there, on 513 x 513 x 128 in FP64.)
 template <typename T, bool EDGE>
 __global__ void __launch_bounds__(256)
-    edge_kernel(const T *__restrict__ C, T *__restrict__ f, T *__restrict__ ch_val,
+    edge_kernel(const T *C, T *__restrict__ f, T *__restrict__ ch_val,
                 const int64_t *__restrict__ ch_start, const int32_t *__restrict__ ch_len,
                 const uint32_t *__restrict__ ch_at, const int32_t *__restrict__ t_idx,
                 const double *__restrict__ t_x, const double *__restrict__ t_y,
@@ -1584,7 +1580,7 @@ cudaError_t launch_edge(const T *C, T *f, T *ch_val, const EdgeTables &t, int64_
 // ------------------------------------------------------------------ moment
 template <typename T>
 __global__ void __launch_bounds__(32 * DR_W)
-    moment_kernel(const T *__restrict__ f, MomentTables mt,
+    moment_kernel(const T *f, MomentTables mt,
                   double *__restrict__ partial, Geometry g) {
   chain_begin();
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1622,7 +1618,7 @@ constexpr int SC_RB = 32;  // r columns per reduction block
 // `count` is a per-handle device counter that the last block resets to 0.
 
 __global__ void __launch_bounds__(SC_THREADS)
-    scan_kernel(const double *__restrict__ partial, MomentTables mt,
+    scan_kernel(const double *partial, MomentTables mt,
                 double *__restrict__ T2, double *__restrict__ bins,
                 double *__restrict__ Mr, double *__restrict__ shift,
                 double *__restrict__ mtot, unsigned int *count, unsigned int *status,
@@ -1735,7 +1731,7 @@ constexpr int ST_U = 16;
 
 template <typename T>
 __global__ void __launch_bounds__(ST_THREADS)
-    stats_kernel(const T *__restrict__ f, const double *__restrict__ R,
+    stats_kernel(const T *f, const double *__restrict__ R,
                  const double *__restrict__ U, const double *__restrict__ J,
                  const double *__restrict__ dR, const double *__restrict__ dU,
                  const double *__restrict__ Ct1, double *__restrict__ part,
@@ -1788,12 +1784,12 @@ __global__ void __launch_bounds__(ST_THREADS)
 
 // block q: quantity q of all block partials, in a fixed order
 __global__ void __launch_bounds__(ST_THREADS)
-    stats_sum_kernel(const double *__restrict__ part, int nblk, double *__restrict__ out4) {
+    stats_sum_kernel(const double *part, int nblk, double *__restrict__ out4) {
   chain_begin();
   const int q = blockIdx.x;
   dd s{0, 0};
   for (int b = threadIdx.x; b < nblk; b += ST_THREADS) {
-    const double2 p = __ldg(reinterpret_cast<const double2 *>(part + (size_t)b * 8) + q);
+    const double2 p = reinterpret_cast<const double2 *>(part + (size_t)b * 8)[q];
     s = dd_add(s, dd{p.x, p.y});
   }
   for (int d = 16; d > 0; d >>= 1) s = dd_add(s, dd_shfl_down(s, d));

@@ -396,8 +396,7 @@ __device__ __forceinline__ void rc2_solve(R (&v)[C::L], const Role &ro, R *dend,
 // values; G receives the u-coefficients.
 template <typename T, typename R, bool KICK, class CF>
 __global__ void __launch_bounds__(CF::NT, CF::MINB)
-    ucol_rc_kernel(const T *__restrict__ f, T *__restrict__ G,
-                   const double *__restrict__ shift, Geometry g,
+    ucol_rc_kernel(const T *f, T *__restrict__ G, const double *shift, Geometry g,
                    const __grid_constant__ RcDir<R> t) {
   constexpr int L = CF::L, LN = CF::LN;
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -423,14 +422,14 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
       uint32_t o = (uint32_t)(kfirst - 1) * nr;
 #pragma unroll
       for (int i = 0; i < L; ++i) {
-        v[i] = (R)__ldg(fc + o);
+        v[i] = (R)fc[o];
         o += nr;
       }
     } else {
 #pragma unroll
       for (int i = 0; i < L; ++i) {
         const int k = min(kfirst + i, N);
-        v[i] = (R)__ldg(fc + (uint32_t)(k - 1) * nr);
+        v[i] = (R)fc[(uint32_t)(k - 1) * nr];
       }
     }
   }
@@ -463,7 +462,7 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
     // unless that fraction is within 1e-9 of a node (then every row takes
     // the exact per-cell path).  Rows with 0 < u + s*hu < N-1 are inside
     // (strictly, vlasovSolver21_spline.hxx:761); outside rows get 0.
-    const double sft = colok ? __ldg(shift + r) : 0.0;
+    const double sft = colok ? shift[r] : 0.0;
     const double qf = sft * g.hu;
     const double fl = floor(qf);
     const double frd = qf - fl;
@@ -590,7 +589,7 @@ __device__ __forceinline__ void cp_async_el(T *smem, const T *gmem) {
 
 template <typename T, typename R, class CF>
 __global__ void __launch_bounds__(CF::NT, CF::MINB)
-    prer_rc_kernel(const T *__restrict__ G, T *__restrict__ C, Geometry g,
+    prer_rc_kernel(const T *G, T *__restrict__ C, Geometry g,
                    const __grid_constant__ RcDir<R> t, unsigned int *err) {
   constexpr int L = CF::L, LN = CF::LN;
   constexpr bool BULK = rc_bulk_rows<CF>();
@@ -709,7 +708,7 @@ constexpr int RC_PIPE_TILES = 4, RC_PIPE_AHEAD = 2;
 
 template <typename T, typename R, class CF>
 __global__ void __launch_bounds__(CF::NT, CF::MINB)
-    prer_pipe_kernel(const T *__restrict__ G, T *__restrict__ C, Geometry g,
+    prer_pipe_kernel(const T *G, T *__restrict__ C, Geometry g,
                      const __grid_constant__ RcDir<R> t, unsigned int *err, int gps,
                      int ngroups) {
   constexpr int L = CF::L, LN = CF::LN;
@@ -1095,9 +1094,9 @@ __device__ __forceinline__ void adj_kick_weights(double fr, double w[4], double 
 //   λ = P_u^T ḡ
 template <typename T, class CF>
 __global__ void __launch_bounds__(CF::NT, CF::MINB)
-    ucol_adj_rc_kernel(const T *__restrict__ f, const double *__restrict__ Gb,
+    ucol_adj_rc_kernel(const T *f, const double *Gb,
                        double *__restrict__ lam, double *__restrict__ sbar,
-                       const double *__restrict__ shift, Geometry g,
+                       const double *shift, Geometry g,
                        const __grid_constant__ RcDir<double> t) {
   chain_begin();
   constexpr int L = CF::L, LN = CF::LN;
@@ -1119,7 +1118,7 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
   {
     const T *fc = f + (size_t)j * N * g.nr + rc;
 #pragma unroll
-    for (int i = 0; i < L; ++i) v[i] = (double)__ldg(fc + (size_t)(min(kfirst + i, N) - 1) * g.nr);
+    for (int i = 0; i < L; ++i) v[i] = (double)fc[(size_t)(min(kfirst + i, N) - 1) * g.nr];
   }
   double c0 = 0.0, cM = 0.0;
   rc_solve<double, CF>(v, ro, E, F, t, c0, cM);
@@ -1148,7 +1147,7 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
   }
   __syncthreads();
   // 3. kick, transposed
-  const double sft = colok ? __ldg(shift + r) : 0.0;
+  const double sft = colok ? shift[r] : 0.0;
   const double qf = sft * g.hu;
   const double fl = floor(qf);
   const double frd = qf - fl;
@@ -1289,7 +1288,7 @@ __global__ void __launch_bounds__(CF::NT, CF::MINB)
 // r lines of the adjoint step: rows of C̄ (all slices) -> P_r^T -> rows of Ḡ
 template <class CF>
 __global__ void __launch_bounds__(CF::NT, CF::MINB)
-    prer_adj_rc_kernel(const double *__restrict__ Cb, double *__restrict__ Gb, Geometry g,
+    prer_adj_rc_kernel(const double *Cb, double *__restrict__ Gb, Geometry g,
                        const __grid_constant__ RcDir<double> t) {
   chain_begin();
   constexpr int L = CF::L, LN = CF::LN;
