@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/vlasolve_b200.h"
+#include "vls_devlist.h"
 #include "vls_hostcopy.h"
 #include "vls_internal.h"
 #include "vls_setup.h"
@@ -44,8 +45,11 @@ struct vls_handle {
   // far-tap cells (their number per slice on the host)
   uint8_t *trip_kinds = nullptr;
   int16_t *win_rows = nullptr;  // window rows of the windowed drift
-  uint32_t *far_base = nullptr, *far_count = nullptr, *far = nullptr;
-  size_t far_cap = 0;
+  uint32_t *far_base = nullptr, *far_count = nullptr;
+  DeviceList<uint32_t> far;
+  // false while the footpoint tables and those that follow them are being
+  // replaced, and after a failure halfway
+  bool foot_ok = false;
   std::vector<uint32_t> far_base_h;
   int64_t nch = 0, nel = 0;
   int64_t *ch_start = nullptr;
@@ -186,6 +190,14 @@ static int dalloc(vls_handle *h, P **p, size_t bytes) {
   return VLS_OK;
 }
 
+// Gives one of the handle's allocations back (nothing may still use it).
+static int dfree(vls_handle *h, void *p, size_t bytes) {
+  h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), p));
+  h->dev_bytes -= bytes;
+  CK(h, cudaFree(p));
+  return VLS_OK;
+}
+
 static int upload(vls_handle *h, void *dst, const void *src, size_t bytes) {
   CK(h, h->copy.upload(dst, src, bytes, h->st));
   CK(h, cudaStreamSynchronize(h->st));
@@ -308,7 +320,8 @@ static uint2 encode_packed(const Coords &c, int32_t code, double rF, double uF) 
   return w;
 }
 
-// The footpoint tables are new: the drift kernels' tables follow them.
+// The footpoint tables are new (foot_ok is false since the first of them was
+// touched): the drift kernels' tables follow them.
 static int footpoints_changed(vls_handle *h) {
   h->fp_gen++;
   const Coords &c = h->co;
@@ -320,13 +333,12 @@ static int footpoints_changed(vls_handle *h) {
                                                      h->st)
                         : launch_window_rows<float>(h->idx, h->fp2, h->win_rows, c.nr, c.nu, c.nj,
                                                     h->st));
+    h->foot_ok = true;
     return VLS_OK;
   }
-  if (!h->trip_kinds) {
-    TRY(dalloc(h, &h->trip_kinds, trip_kinds_bytes(c.nr, c.nu, c.nj)));
-    TRY(dalloc(h, &h->far_count, sizeof(uint32_t) * c.nj));
-    TRY(dalloc(h, &h->far_base, sizeof(uint32_t) * (c.nj + 1)));
-  }
+  if (!h->trip_kinds) TRY(dalloc(h, &h->trip_kinds, trip_kinds_bytes(c.nr, c.nu, c.nj)));
+  if (!h->far_count) TRY(dalloc(h, &h->far_count, sizeof(uint32_t) * c.nj));
+  if (!h->far_base) TRY(dalloc(h, &h->far_base, sizeof(uint32_t) * (c.nj + 1)));
   CK(h, launch_trip_kinds(h->fp2, h->trip_kinds, c.nr, c.nu, c.nj, h->st));
   CK(h, launch_far_cells(h->fp2, nullptr, h->far_count, nullptr, c.nr, c.nu, c.nj, h->st));
   CK(h, cudaMemcpyAsync(h->far_base_h.data() + 1, h->far_count, sizeof(uint32_t) * c.nj,
@@ -338,14 +350,14 @@ static int footpoints_changed(vls_handle *h) {
     if (total > 0xffffffffu) return fail(h, VLS_EINVAL, "too many far footpoints");
     h->far_base_h[j + 1] = (uint32_t)total;
   }
-  if (total > h->far_cap || !h->far) {
-    // grown for footpoints with more such cells (an outgrown list is freed
-    // with the handle)
-    h->far_cap = total;
-    TRY(dalloc(h, &h->far, sizeof(uint32_t) * std::max<size_t>(total, 1)));
-  }
+  // (the stream was just waited for: no step still reads an outgrown list)
+  TRY(h->far.reserve(
+      std::max<size_t>(total, 1),
+      [&](uint32_t **q, size_t n) { return dalloc(h, q, sizeof(uint32_t) * n); },
+      [&](uint32_t *q, size_t n) { return dfree(h, q, sizeof(uint32_t) * n); }));
   TRY(upload(h, h->far_base, h->far_base_h.data(), sizeof(uint32_t) * (c.nj + 1)));
-  CK(h, launch_far_cells(h->fp2, h->far_base, nullptr, h->far, c.nr, c.nu, c.nj, h->st));
+  CK(h, launch_far_cells(h->fp2, h->far_base, nullptr, h->far.p, c.nr, c.nu, c.nj, h->st));
+  h->foot_ok = true;
   return VLS_OK;
 }
 
@@ -1108,6 +1120,7 @@ extern "C" int vls_set_footpoints(vls_handle *h, const int32_t *rI,
       idx[i] = rI[i] | (uI[i] << 16);
     }
   }
+  h->foot_ok = false;
   if (h->prec == VLS_FP64) {
     TRY(upload(h, h->idx, idx.data(), sizeof(int32_t) * h->cells));
     TRY(upload(h, h->fx, rF, sizeof(double) * h->cells));
@@ -1132,6 +1145,14 @@ const RcDir<float> &rcdir<float>(const vls_handle *h, bool u) {
   return u ? h->rcu_f : h->rcr_f;
 }
 
+// A failed vls_set_footpoints leaves words, trip kinds, window rows and far
+// cells of different footpoints; a step over them would keep stale values.
+static int check_footpoints(vls_handle *h) {
+  if (h->foot_ok) return VLS_OK;
+  return fail(h, VLS_ESTATE, "the footpoint tables are incomplete after a failed "
+                             "vls_set_footpoints: set them again");
+}
+
 // One split step: f_out = D P_r P_u Kick(P_u f_in).  f_in, f_out and the
 // kick's shift are the handle's unless given (the adjoint's recomputation
 // steps from one stored state into the next with the shift it stored); f_in
@@ -1139,6 +1160,7 @@ const RcDir<float> &rcdir<float>(const vls_handle *h, bool u) {
 template <typename T, typename R>
 static int drift_once(vls_handle *h, bool kick, const void *f_in = nullptr,
                       void *f_out = nullptr, const double *shift = nullptr) {
+  TRY(check_footpoints(h));
   const T *fin = (const T *)(f_in ? f_in : h->f);
   T *fout = (T *)(f_out ? f_out : h->f);
   const double *sft = shift ? shift : h->shift;
@@ -1186,7 +1208,7 @@ static int drift_once(vls_handle *h, bool kick, const void *f_in = nullptr,
                                          (int64_t)(h->far_base_h[j + 1] - h->far_base_h[j]));
     if (most > 0) {
       const EdgeTables et{h->ch_start, h->ch_len,      h->ch_at,    h->t_idx, h->t_x,
-                          h->t_y,      h->d_chain_lo, h->far_base, h->far};
+                          h->t_y,      h->d_chain_lo, h->far_base, h->far.p};
       CK(h, timed(
                 h, VLS_K_TAILS,
                 [&] {
@@ -1685,6 +1707,7 @@ static bool adj_entry_ordered(vls_handle *h) {
 
 template <typename T>
 static int ensure_inv(vls_handle *h) {
+  TRY(check_footpoints(h));
   if (h->inv_gen == h->fp_gen) return VLS_OK;
   const Geometry g = geometry(h);
   const int64_t nch = h->nch;
