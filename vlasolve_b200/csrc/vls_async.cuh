@@ -123,9 +123,17 @@ __device__ __forceinline__ void bulk_wait_read() {
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-template <typename... P, typename... A>
+// Each argument converts to its parameter implicitly (the kernel alone names
+// the parameter types), as in a <<<>>> launch: no pointer passes for another
+// type's.  Returns the launch's error, and leaves none behind for the next
+// cudaGetLastError of an unrelated call.
+template <typename P>
+struct ChainArg {
+  using type = P;
+};
+template <typename... P>
 inline cudaError_t chain_launch(void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
-                                cudaStream_t st, A &&...args) {
+                                cudaStream_t st, const typename ChainArg<P>::type &...args) {
   cudaLaunchConfig_t c = {};
   c.gridDim = grid;
   c.blockDim = block;
@@ -136,7 +144,9 @@ inline cudaError_t chain_launch(void (*kern)(P...), dim3 grid, dim3 block, size_
   at[0].val.programmaticStreamSerializationAllowed = 1;
   c.attrs = at;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kern, P(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kern, args...);
+  const cudaError_t last = cudaGetLastError();
+  return e != cudaSuccess ? e : last;
 }
 
 }  // namespace vls
