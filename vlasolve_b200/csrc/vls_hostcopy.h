@@ -14,11 +14,10 @@
 #include <cstdint>
 #include <cstring>
 #include <mutex>
-#include <vector>
 
 namespace vls {
 
-// memcpy by all host threads, in pieces of whole pages of the destination
+// memcpy by all host threads, in pieces of many pages
 inline void parallel_copy(void *dst, const void *src, size_t n) {
   const size_t piece = (size_t)256 << 10;
   const int64_t np = (int64_t)((n + piece - 1) / piece);
@@ -48,33 +47,31 @@ class ChunkPool {
     std::lock_guard<std::mutex> lk(m_);
     users_ += d;
     if (users_ == 0) {
-      for (Pair &q : free_) drop(q);
-      free_.clear();
+      while (nfree_) drop(free_[--nfree_]);
     }
   }
-  cudaError_t take(Pair &q) {
+  // false where no memory can be page-locked (the copy then goes without)
+  bool take(Pair &q) {
     {
       std::lock_guard<std::mutex> lk(m_);
-      if (!free_.empty()) {
-        q = free_.back();
-        free_.pop_back();
-        return cudaSuccess;
+      if (nfree_) {
+        q = free_[--nfree_];
+        return true;
       }
     }
-    for (int k = 0; k < 2; ++k) {
-      const cudaError_t e = cudaHostAlloc(&q.p[k], CHUNK, cudaHostAllocPortable);
-      if (e != cudaSuccess) {
+    for (int k = 0; k < 2; ++k)
+      if (cudaHostAlloc(&q.p[k], CHUNK, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
         q.p[k] = nullptr;
         drop(q);
-        return e;
+        return false;
       }
-    }
-    return cudaSuccess;
+    return true;
   }
   void give(Pair &q) {
     std::lock_guard<std::mutex> lk(m_);
-    if (free_.size() < KEEP)
-      free_.push_back(q);
+    if (nfree_ < KEEP)
+      free_[nfree_++] = q;
     else
       drop(q);
   }
@@ -87,7 +84,8 @@ class ChunkPool {
     }
   }
   std::mutex m_;
-  std::vector<Pair> free_;
+  Pair free_[KEEP];
+  size_t nfree_ = 0;
   int users_ = 0;
 };
 
@@ -105,9 +103,10 @@ class HostCopy {
   HostCopy &operator=(const HostCopy &) = delete;
 
   cudaError_t download(void *host, const void *dev, size_t bytes, cudaStream_t st) {
-    if (!staged(host, bytes))
+    ChunkPool::Pair q;
+    if (!staged(host, bytes) || !ChunkPool::get().take(q))
       return cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, st);
-    return run(bytes, st, [&](size_t o, size_t n, void *chunk, int phase) {
+    return run(q, bytes, st, [&](size_t o, size_t n, void *chunk, int phase) {
       if (phase == 0)
         return cudaMemcpyAsync(chunk, (const char *)dev + o, n, cudaMemcpyDeviceToHost, st);
       parallel_copy((char *)host + o, chunk, n);
@@ -115,9 +114,10 @@ class HostCopy {
     }, false);
   }
   cudaError_t upload(void *dev, const void *host, size_t bytes, cudaStream_t st) {
-    if (!staged(host, bytes))
+    ChunkPool::Pair q;
+    if (!staged(host, bytes) || !ChunkPool::get().take(q))
       return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, st);
-    return run(bytes, st, [&](size_t o, size_t n, void *chunk, int phase) {
+    return run(q, bytes, st, [&](size_t o, size_t n, void *chunk, int phase) {
       if (phase == 0) {
         parallel_copy(chunk, (const char *)host + o, n);
         return cudaMemcpyAsync((char *)dev + o, chunk, n, cudaMemcpyHostToDevice, st);
@@ -147,16 +147,15 @@ class HostCopy {
   // chunk k: phase 0 queues its copy, phase 1 comes when that copy is done.
   // Two chunks alternate; both copies are done on return.
   template <typename F>
-  cudaError_t run(size_t bytes, cudaStream_t st, F &&f, bool up) {
+  cudaError_t run(ChunkPool::Pair &q, size_t bytes, cudaStream_t st, F &&f, bool up) {
     constexpr size_t C = ChunkPool::CHUNK;
     cudaError_t e = cudaSuccess;
     for (cudaEvent_t &ev : ev_)
       if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess) {
         ev = nullptr;
+        ChunkPool::get().give(q);
         return e;
       }
-    ChunkPool::Pair q;
-    if ((e = ChunkPool::get().take(q)) != cudaSuccess) return e;
     const size_t n = (bytes + C - 1) / C;
     auto done = [&](size_t k) {
       cudaError_t r = cudaEventSynchronize(ev_[k & 1]);
