@@ -670,24 +670,23 @@ __device__ __forceinline__ Cell<double> decode(const RawCell<double> &r) {
   return c;
 }
 
-// 4x4 gather from a shared window row-pitched DW_COLS (immediate offsets)
-template <typename T>
-__device__ __forceinline__ T eval_window(const T *p, T x, T y) {
+// 4x4 gather from a shared window of row pitch PITCH (immediate offsets)
+template <int PITCH, typename T>
+__device__ __forceinline__ T eval_pitch(const T *p, T x, T y) {
   const T b2xI = bv2<T>(T(1) - x), b1xI = bv1<T>(T(1) - x);
   const T b1x = bv1<T>(x), b2x = bv2<T>(x);
   const T s0 = p[0] * b2xI + p[1] * b1xI + p[2] * b1x + p[3] * b2x;
-  const T s1 = p[DW_COLS] * b2xI + p[DW_COLS + 1] * b1xI + p[DW_COLS + 2] * b1x +
-               p[DW_COLS + 3] * b2x;
-  const T s2 = p[2 * DW_COLS] * b2xI + p[2 * DW_COLS + 1] * b1xI +
-               p[2 * DW_COLS + 2] * b1x + p[2 * DW_COLS + 3] * b2x;
-  const T s3 = p[3 * DW_COLS] * b2xI + p[3 * DW_COLS + 1] * b1xI +
-               p[3 * DW_COLS + 2] * b1x + p[3 * DW_COLS + 3] * b2x;
+  const T s1 = p[PITCH] * b2xI + p[PITCH + 1] * b1xI + p[PITCH + 2] * b1x + p[PITCH + 3] * b2x;
+  const T s2 = p[2 * PITCH] * b2xI + p[2 * PITCH + 1] * b1xI + p[2 * PITCH + 2] * b1x +
+               p[2 * PITCH + 3] * b2x;
+  const T s3 = p[3 * PITCH] * b2xI + p[3 * PITCH + 1] * b1xI + p[3 * PITCH + 2] * b1x +
+               p[3 * PITCH + 3] * b2x;
   return over36<T>(bv2<T>(T(1) - y) * s0 + bv1<T>(T(1) - y) * s1 +
                            bv1<T>(y) * s2 + bv2<T>(y) * s3);
 }
-template <>
-__device__ __forceinline__ float eval_window<float>(const float *p, float x, float y) {
-  return gather_f32x2([&](int a, int b) { return p[a * DW_COLS + b]; }, x, y);
+template <int PITCH>
+__device__ __forceinline__ float eval_pitch(const float *p, float x, float y) {
+  return gather_f32x2([&](int a, int b) { return p[a * PITCH + b]; }, x, y);
 }
 
 constexpr int DW_MAX_CH = 2048 / DW_CH;   // chunks of the tallest slice
@@ -859,7 +858,7 @@ __global__ void __launch_bounds__(DT_THREADS)
         if (cl.kind == 0) {
           const int wr = cl.uI - y0, wc = cl.rI - x0;
           if (have && wr >= 0 && wr <= DW_ROWS - 4 && wc >= 0 && wc <= DW_COLS - 4)
-            v = eval_window<T>(wb + wr * DW_COLS + wc, cl.x, cl.y);
+            v = eval_pitch<DW_COLS>(wb + wr * DW_COLS + wc, cl.x, cl.y);
           else
             v = eval2d<T>(Cj, g.pc, cl.rI, cl.x, cl.uI, cl.y);
         } else if (cl.kind == 2) {
@@ -932,11 +931,6 @@ cudaError_t launch_drift_tma(const CUtensorMap *tmC, const T *C, T *f, const int
 // reach hundreds of rows while their r displacements stay within a few
 // columns.  Cells whose taps leave the strip's columns gather from global
 // memory.
-template <int PITCH>
-__device__ __forceinline__ float eval_pitch_f32x2(const float *p, float x, float y) {
-  return gather_f32x2([&](int a, int b) { return p[a * PITCH + b]; }, x, y);
-}
-
 // The kinds of a trip, DS_TRIP rows of one strip (32 columns) of a slice:
 // nothing to compute (every cell outside the box: 0), regular (every cell
 // gathers inside the strip, and from row to row each column's 4 x 4 taps move
@@ -1159,7 +1153,7 @@ __device__ __forceinline__ double strip_trip(bool regular, const float *win, con
       float edge = 0.f;
       if (!in && c[h].x != FP_OUT && row) edge = o[h * nr];
       const float2 xy = frac21x2(c[h]);
-      v[h] = eval_pitch_f32x2<WC>(win + (in ? (c[h].y >> FP_FBITS) * WC + wc : 0u), xy.x, xy.y);
+      v[h] = eval_pitch<WC>(win + (in ? (c[h].y >> FP_FBITS) * WC + wc : 0u), xy.x, xy.y);
       v[h] = in ? v[h] : edge;
       if (row)
         o[h * nr] = v[h];
@@ -1174,14 +1168,15 @@ __device__ __forceinline__ double strip_trip(bool regular, const float *win, con
 
 // Shared memory of the strip drift: NB strip buffers (nch boxes of `rows`
 // rows), then per buffer the column sums of every warp and the trips' kinds,
-// then the moment weights.  The boxes hold N_u + 3 rows with as little excess
-// as even heights of at most 256 rows give (16-byte-multiple boxes on
-// 128-byte boundaries).
+// then the moment weights where they fit (else they are read in global
+// memory: strips of 568 .. 573 rows with two buffers, 1148 and 1149 with one).
+// The boxes hold N_u + 3 rows with as little excess as even heights of at most
+// 256 rows give (16-byte-multiple boxes on 128-byte boundaries).
 struct StripSmem {
   size_t strip, red, kinds, total;  // bytes: one buffer's parts, everything
   int nch, rows, nt;
 };
-__host__ __device__ inline StripSmem strip_smem(int nu, int nw, int nb) {
+__host__ __device__ inline StripSmem strip_smem(int nu, int nw, int nb, bool weights) {
   StripSmem s;
   s.nch = (nu + 3 + 255) / 256;
   s.rows = (nu + 3 + 2 * s.nch - 1) / (2 * s.nch) * 2;
@@ -1189,10 +1184,11 @@ __host__ __device__ inline StripSmem strip_smem(int nu, int nw, int nb) {
   s.strip = (size_t)s.nch * s.rows * DS_WC * sizeof(float);
   s.red = ((size_t)nw * 33 * sizeof(double) + 15) / 16 * 16;
   s.kinds = (size_t)(s.nt + 15) / 16 * 16;
-  s.total = nb * (s.strip + s.red + s.kinds) + (size_t)s.nt * DS_TRIP * sizeof(float);
+  s.total = nb * (s.strip + s.red + s.kinds) +
+            (weights ? (size_t)s.nt * DS_TRIP * sizeof(float) : 0);
   return s;
 }
-int drift_strip_box_rows(int nu) { return strip_smem(nu, 1, 1).rows; }
+
 
 // Block: NW consumer warps and a producer warp; persistent, a task being one
 // strip (32 output columns) of one J slice.  The producer keeps NB strips
@@ -1219,7 +1215,7 @@ int drift_strip_box_rows(int nu) { return strip_smem(nu, 1, 1).rows; }
 // polls) gathers that strip's cells from global memory; the producer waits
 // (full limit) for a strip's own boxes before it refills its buffer and
 // before the block ends, whatever the consumers did.
-template <int NW, int NB, int MINB>
+template <int NW, int NB, int MINB, bool WEIGHTS>
 __global__ void __launch_bounds__(32 * (NW + 1), MINB)
     drift_strip_kernel(const __grid_constant__ CUtensorMap tmS, const float *C,
                        float *f, const uint2 *__restrict__ fp2,
@@ -1229,12 +1225,13 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
   constexpr int WC = DS_WC;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint64_t full[NB], done[NB];
-  const StripSmem L = strip_smem(g.nu, NW, NB);
+  const StripSmem L = strip_smem(g.nu, NW, NB, WEIGHTS);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int ns = strip_blocks(g.nr), ntask = ns * g.nb, nt = L.nt;
   const bool extra = ns * 32 < g.nr;  // the last strip also takes the last column
   unsigned char *kinds0 = smem_raw + NB * (L.strip + L.red);
-  float *bus = reinterpret_cast<float *>(kinds0 + NB * L.kinds);
+  float *wsm = reinterpret_cast<float *>(kinds0 + NB * L.kinds);
+  const float *bus = WEIGHTS ? wsm : mt.bu32;
   auto buf_win = [&](int b) { return reinterpret_cast<float *>(smem_raw + b * L.strip); };
   auto buf_red = [&](int b) {
     return reinterpret_cast<double *>(smem_raw + NB * L.strip + b * L.red);
@@ -1247,7 +1244,8 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
     mbar_fence_init();
   }
   chain_begin();
-  for (int u = tid; u < nt * DS_TRIP; u += 32 * (NW + 1)) bus[u] = __ldg(mt.bu32 + u);
+  if constexpr (WEIGHTS)
+    for (int u = tid; u < nt * DS_TRIP; u += 32 * (NW + 1)) wsm[u] = __ldg(mt.bu32 + u);
   __syncthreads();
   const int nmine = (int)blockIdx.x < ntask ? (ntask - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
@@ -1438,7 +1436,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
         const uint2 c = __ldg(fp2 + cell);
         float v = 0.f;
         if (ok && in_strip(c, x0))
-          v = eval_pitch_f32x2<WC>(
+          v = eval_pitch<WC>(
               win + (c.y >> FP_FBITS) * WC + ((c.x >> FP_FBITS) - (uint32_t)x0), frac21(c.x),
               frac21(c.y));
         else if (c.x < FP_CHAIN)
@@ -1472,47 +1470,56 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
 // DRIFT_WINDOW: none, the windowed kernel.  `want` != DRIFT_AUTO asks for
 // one kind, returned only if it fits (else DRIFT_WINDOW).  FP64 takes the
 // windowed kernel.
+static bool strip_fits(int nu, int nb, bool weights) {
+  // 227 KB of shared memory per block with the barriers; strips of 576 and
+  // 1152 rows at most (taller ones, which would fit without the weights, have
+  // been measured with windows only)
+  return nu + 3 <= 1152 / nb && strip_smem(nu, STRIP_WARPS, nb, weights).total + 256 <= 232448;
+}
 template <typename T>
 int drift_strip_width(int nu, int want) {
   if (sizeof(T) != 4 || want == DRIFT_WINDOW) return DRIFT_WINDOW;
-  // 227 KB of shared memory per block, the barriers' 1 KB kept free
-  const bool fit2 = strip_smem(nu, STRIP_WARPS, 2).total + 1024 <= 232448;
-  const bool fit1 = strip_smem(nu, STRIP_WARPS, 1).total + 1024 <= 232448;
+  const bool fit2 = strip_fits(nu, 2, false), fit1 = strip_fits(nu, 1, false);
   if (want == DRIFT_STRIP2) return fit2 ? DRIFT_STRIP2 : DRIFT_WINDOW;
   if (want == DRIFT_STRIP1) return fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
   return fit2 ? DRIFT_STRIP2 : fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
 }
+int drift_strip_box_rows(int nu) { return strip_smem(nu, 1, 1, false).rows; }
 
-template <int NW, int NB, int MINB>
+template <int NW, int NB, int MINB, bool WEIGHTS>
 static cudaError_t drift_strip_go(const CUtensorMap *tmS, const float *C, float *f,
                                   const uint2 *fp2, const uint8_t *trip_kinds,
                                   const MomentTables &mt, double *partial, unsigned int *err,
                                   uint32_t spins, const Geometry &g, cudaStream_t st) {
-  const size_t smem = strip_smem(g.nu, NW, NB).total;
-  cudaError_t e = cudaFuncSetAttribute(drift_strip_kernel<NW, NB, MINB>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = strip_smem(g.nu, NW, NB, WEIGHTS).total;
+  auto kern = drift_strip_kernel<NW, NB, MINB, WEIGHTS>;
+  cudaError_t e =
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   int dev = 0, nsm = 0;
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return e;
   const int ntask = strip_blocks(g.nr) * g.nb;
-  return chain_launch(drift_strip_kernel<NW, NB, MINB>, dim3(std::min(ntask, nsm * MINB)),
-                      dim3(32 * (NW + 1)), smem, st, *tmS, C, f, fp2, trip_kinds, mt, partial, err,
-                      spins, g);
+  return chain_launch(kern, dim3(std::min(ntask, nsm * MINB)), dim3(32 * (NW + 1)), smem, st, *tmS,
+                      C, f, fp2, trip_kinds, mt, partial, err, spins, g);
 }
 
 cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C, float *f,
                                const uint2 *fp2, const uint8_t *trip_kinds,
                                const MomentTables &mt, double *partial, unsigned int *err,
                                uint32_t spins, const Geometry &g, cudaStream_t st) {
+  auto go = [&](auto with, auto without, int nb) {
+    return (strip_fits(g.nu, nb, true) ? with : without)(tmS, C, f, fp2, trip_kinds, mt, partial,
+                                                         err, spins, g, st);
+  };
   switch (kind) {
     case DRIFT_STRIP2:
-      return drift_strip_go<STRIP_WARPS, 2, 1>(tmS, C, f, fp2, trip_kinds, mt, partial, err,
-                                               spins, g, st);
+      return go(drift_strip_go<STRIP_WARPS, 2, 1, true>, drift_strip_go<STRIP_WARPS, 2, 1, false>,
+                2);
     case DRIFT_STRIP1:
-      return drift_strip_go<STRIP_WARPS, 1, 1>(tmS, C, f, fp2, trip_kinds, mt, partial, err,
-                                               spins, g, st);
+      return go(drift_strip_go<STRIP_WARPS, 1, 1, true>, drift_strip_go<STRIP_WARPS, 1, 1, false>,
+                1);
     default:
       return cudaErrorInvalidValue;
   }
