@@ -125,7 +125,7 @@ int vls_create(const vls_grid_desc *grid, const vls_solver_desc *solver,
                        else one), FP64 storage and strips too tall for one
                        block take staged windows; VLS_DRIFT_WINDOW /
                        _STRIP2 / _STRIP1 ask for one of those (a strip that
-                       does not fit, or FP64, falls back to windows).
+                       does not fit falls back to windows).
      slices_per_batch  J slices per batch of the prefilter and drift scratch
                        (0: all slices in one batch); the G and C scratch
                        holds streams x slices_per_batch slices.

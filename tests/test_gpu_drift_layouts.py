@@ -1,4 +1,5 @@
-"""Drift layouts that a handle asks for, at the edges of what fits: FP32 strips
+"""Drift layouts that a handle asks for, at the edges of what fits: FP64 strips
+(two blocks of up to 253 v_r vertices per SM, one of up to 573), FP32 strips
 (two buffers up to 573 vertices, one up to 1149; the tallest of each read the
 moment weights in global memory), windows beyond.  Against the oracle, FP64 to
 1e-12 of the largest value, FP32 to the storage modes' bounds (relative L2
@@ -31,6 +32,10 @@ def _close(s, o, precision):
 
 
 @pytest.mark.parametrize("precision,want,nr,nu,drift", [
+    ("fp64", "strip2", 65, 33, "strip2"), ("fp64", "strip1", 65, 33, "strip1"),
+    ("fp64", "strip2", 41, 253, "strip2"), ("fp64", "strip2", 41, 254, "window"),
+    ("fp64", "strip1", 41, 254, "strip1"), ("fp64", "strip1", 33, 573, "strip1"),
+    ("fp64", "strip1", 33, 574, "window"), ("fp64", "strip1", 9, 8, "strip1"),
     ("fp64", "auto", 65, 33, "window"),
     ("fp32", "strip2", 41, 567, "strip2"), ("fp32", "strip2", 65, 568, "strip2"),
     ("fp32", "auto", 41, 573, "strip2"), ("fp32", "auto", 41, 574, "strip1"),
@@ -49,3 +54,32 @@ def test_layout_is_the_one_asked_for(precision, want, nr, nu, drift):
         o.step(1)
         _close(s, o, precision)
     s.sync()
+
+
+@pytest.mark.parametrize("drift", ["strip2", "strip1"])
+def test_fp64_strip_wait_timeout_reports_and_falls_back(drift):
+    """Waits that give up at once: reported, and the cells read C in global
+    memory (the copies still land before the block ends)."""
+    from vlasolve_b200 import VlasovSolver21Spline, _lib
+    cfg = _cfg(65, 33)
+    s = VlasovSolver21Spline(cfg, precision="fp64",
+                             layout={"drift": drift, "drift_wait_spins": -1})
+    o = Oracle(cfg)
+    s.step(1)
+    o.step(1)
+    with pytest.raises(_lib.VlsError) as e:
+        s.sync()
+    assert e.value.code == _lib.VLS_ECUDA and "drift" in str(e.value)
+    _close(s, o, "fp64")
+
+
+@pytest.mark.parametrize("drift", ["strip2", "strip1"])
+def test_fp64_strips_in_batches_are_bit_identical(drift):
+    from vlasolve_b200 import VlasovSolver21Spline
+    cfg = _cfg(65, 70)
+    a = VlasovSolver21Spline(cfg, precision="fp64", layout={"drift": drift})
+    b = VlasovSolver21Spline(cfg, precision="fp64",
+                             layout={"drift": drift, "slices_per_batch": 2, "streams": 2})
+    a.step(4)
+    b.step(4)
+    np.testing.assert_array_equal(a.f, b.f)

@@ -326,6 +326,10 @@ static int footpoints_changed(vls_handle *h) {
   h->fp_gen++;
   const Coords &c = h->co;
   h->far_base_h.assign((size_t)c.nj + 1, 0);
+  if (h->esize == 8 && h->drift_kind != DRIFT_WINDOW) {
+    h->foot_ok = true;  // FP64 strips test every cell
+    return VLS_OK;
+  }
   if (h->drift_kind == DRIFT_WINDOW) {
     if (!h->win_rows)
       TRY(dalloc(h, &h->win_rows, sizeof(int16_t) * window_rows_count(c.nr, c.nu, c.nj)));
@@ -553,9 +557,13 @@ static bool make_tensor_map(vls_handle *h) {
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return false;
     if (h->drift_kind != DRIFT_WINDOW) {
-      const cuuint32_t sbox[3] = {48, (cuuint32_t)drift_strip_box_rows(h->co.nu), 1};
-      if (enc(&h->tmS[s], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, sbox, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+      const cuuint32_t sbox[3] = {48,
+                                  (cuuint32_t)(es == 4 ? drift_strip_box_rows<float>(h->co.nu)
+                                                       : drift_strip_box_rows<double>(h->co.nu)),
+                                  1};
+      if (enc(&h->tmS[s],
+              es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
+              base, dims, strides, sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) !=
           CUDA_SUCCESS)
         return false;
@@ -1220,7 +1228,13 @@ static int drift_once(vls_handle *h, bool kick, const void *f_in = nullptr,
     CK(h, timed(
               h, VLS_K_DRIFT,
               [&] {
-                if constexpr (sizeof(T) == 4) {
+                if constexpr (sizeof(T) == 8) {
+                  if (h->drift_kind != DRIFT_WINDOW)
+                    return launch_drift_strip64(
+                        &h->tmS[sl], h->drift_kind, C, fout, h->idx, (const T *)h->fx,
+                        (const T *)h->fy, h->ch_start, h->ch_len, (const T *)h->ch_val, h->ndrift,
+                        moment_tables(h), h->partial, h->flag + 1, h->drift_spins, g, bs);
+                } else {
                   if (h->drift_kind != DRIFT_WINDOW)
                     return launch_drift_strip(&h->tmS[sl], h->drift_kind, C, fout, h->fp2,
                                               h->trip_kinds, moment_tables(h), h->partial,

@@ -1465,11 +1465,131 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
   }
 }
 
-// Strip layouts (the DRIFT_* kinds), FP32 storage: DRIFT_STRIP2, two strip
-// buffers per block; DRIFT_STRIP1, one (strips too tall for two);
-// DRIFT_WINDOW: none, the windowed kernel.  `want` != DRIFT_AUTO asks for
-// one kind, returned only if it fits (else DRIFT_WINDOW).  FP64 takes the
-// windowed kernel.
+// FP64 strips, for handles that ask for them (VLS_DRIFT_STRIP2 / _STRIP1; the
+// windowed drift is the faster one and FP64's default: 513 x 513 x 128
+// Hernquist STRIP1 0.358 ms against 0.301, 257 x 253 x 128 STRIP2 0.100
+// against 0.095).  Block: 32 output columns x every row of one J slice; the
+// whole strip is staged in boxes of D64_ROWS rows, lanes walk the rows of a
+// column in turn, footpoints two rows ahead; cells whose taps leave the strip,
+// chain fronts and, after a wait that ran out, every cell are read in global
+// memory.
+constexpr int D64_ROWS = 64, D64_AHEAD = 2;
+template <int NW, int MINB>
+__global__ void __launch_bounds__(32 * NW, MINB)
+    drift_strip64_kernel(const __grid_constant__ CUtensorMap tmS, const double *C,
+                         double *__restrict__ f, const int32_t *__restrict__ idx,
+                         const double *__restrict__ fx, const double *__restrict__ fy,
+                         const int64_t *__restrict__ ch_start,
+                         const int32_t *__restrict__ ch_len, const double *ch_val,
+                         int64_t ndrift, MomentTables mt, double *__restrict__ partial,
+                         unsigned int *err, uint32_t spins, Geometry g) {
+  constexpr int WC = DS_WC, PF = D64_AHEAD;
+  static_assert(NW * PF + 1 <= FOOT_PAD_ROWS, "the loads ahead reach past the padding rows");
+  constexpr uint32_t BYTES = D64_ROWS * WC * sizeof(double);
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ double red[NW][32];
+  const int rows = g.nu + 3, nch = (rows + D64_ROWS - 1) / D64_ROWS;
+  double *win = reinterpret_cast<double *>(smem_raw);
+  uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + (size_t)nch * BYTES);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int r0 = blockIdx.x * 32, r = r0 + lane, x0 = r0 - DS_XL;
+  const int jl = blockIdx.y, j = g.j0 + jl;
+  const bool col_ok = r < g.nr;
+  chain_begin();
+  if (tid == 0) {
+    for (int c = 0; c < nch; ++c) mbar_init(&bar[c], 1);
+    mbar_fence_init();
+    for (int c = 0; c < nch; ++c) {
+      mbar_expect_tx(&bar[c], BYTES);
+      tma_load_3d(win + (size_t)c * D64_ROWS * WC, &tmS, x0, c * D64_ROWS, jl, &bar[c]);
+    }
+  }
+  __syncthreads();
+  const double *Cj = C + (size_t)jl * rows * g.pc;
+  bool staged = true;
+  for (int c = 0; c < nch && staged; ++c) staged = mbar_wait_bounded(&bar[c], 0u, spins);
+  if (!staged) atomicOr(err, 1u);
+  auto value = [&](const RawCell<double> &c) {
+    const Cell<double> cl = decode(c);
+    if (cl.kind == 0) {
+      const uint32_t wc = (uint32_t)(cl.rI - x0);
+      if (staged && wc < (uint32_t)(WC - 3))
+        return eval_pitch<WC>(win + cl.uI * WC + wc, cl.x, cl.y);
+      return eval2d<double>(Cj, g.pc, cl.rI, cl.x, cl.uI, cl.y);
+    }
+    if (cl.kind == 2) return ch_val[__ldg(ch_start + cl.ch) + ndrift % __ldg(ch_len + cl.ch)];
+    return 0.0;
+  };
+  // rows w, w + NW, ...; loads ahead run past the slice into the next one or
+  // the tables' padding, and lanes past N_r read the next row's words
+  const size_t sb = (size_t)j * g.nu * g.nr;
+  const uint32_t step = (uint32_t)NW * (uint32_t)g.nr;
+  uint32_t off = (uint32_t)w * (uint32_t)g.nr + (uint32_t)r;
+  RawCell<double> q[PF];
+#pragma unroll
+  for (int k = 0; k < PF; ++k) q[k] = load_raw(idx + sb, fx + sb, fy + sb, nullptr, off + k * step);
+  double acc = 0.0;
+  for (int u = w; u < g.nu; u += NW * PF) {
+    double part = 0.0;
+#pragma unroll
+    for (int k = 0; k < PF; ++k) {
+      const RawCell<double> c = q[k];
+      if (u + NW * k < g.nu)
+        q[k] = load_raw(idx + sb, fx + sb, fy + sb, nullptr, off + PF * step);
+      if (u + NW * k < g.nu && col_ok) {
+        const double v = value(c);
+        f[sb + off] = v;
+        part += __ldg(mt.bu + u + NW * k) * v;
+      }
+      off += step;
+    }
+    acc += part;
+  }
+  // N_r = 32 k + 1: the last block also takes the last column, one row per
+  // thread (its strip covers columns r0 - 8 .. r0 + 39)
+  const bool extra = (int)gridDim.x * 32 < g.nr && blockIdx.x == gridDim.x - 1;
+  double acc2 = 0.0;
+  if (extra)
+    for (int u = tid; u < g.nu; u += 32 * NW) {
+      const size_t cell = sb + (size_t)u * g.nr + r0 + 32;
+      const double v = value(load_raw(idx, fx, fy, nullptr, cell));
+      f[cell] = v;
+      acc2 += __ldg(mt.bu + u) * v;
+    }
+  // every box must have landed before the block's shared memory is released
+  if (tid == 0)
+    for (int c = 0; c < nch; ++c)
+      if (!mbar_wait_bounded(&bar[c], 0u)) atomicOr(err, 2u);
+  red[w][lane] = acc;
+  __syncthreads();
+  if (w == 0 && col_ok) {
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < NW; ++k) sum += red[k][lane];
+    partial[(size_t)j * g.nr + r] = __ldg(mt.wj + j) * sum;
+  }
+  if (extra) {
+    __syncthreads();
+    red[w][lane] = acc2;
+    __syncthreads();
+    if (tid == 0) {
+      double sum = 0.0;
+      for (int k = 0; k < NW; ++k)
+        for (int l = 0; l < 32; ++l) sum += red[k][l];
+      partial[(size_t)j * g.nr + r0 + 32] = __ldg(mt.wj + j) * sum;
+    }
+  }
+}
+
+// Strip layouts (the DRIFT_* kinds).  FP32: DRIFT_STRIP2, two strip buffers
+// per block; DRIFT_STRIP1, one (strips too tall for two).  FP64: DRIFT_STRIP2,
+// two blocks of one strip per SM; DRIFT_STRIP1, one.  DRIFT_WINDOW: none, the
+// windowed kernel, which FP64 takes unless a strip is asked for.  `want` !=
+// DRIFT_AUTO asks for one kind, returned only if it fits (else DRIFT_WINDOW).
+static size_t strip64_smem(int nu) {
+  const int nch = (nu + 3 + D64_ROWS - 1) / D64_ROWS;
+  return (size_t)nch * (D64_ROWS * DS_WC * sizeof(double) + sizeof(uint64_t));
+}
 static bool strip_fits(int nu, int nb, bool weights) {
   // 227 KB of shared memory per block with the barriers; strips of 576 and
   // 1152 rows at most (taller ones, which would fit without the weights, have
@@ -1478,13 +1598,25 @@ static bool strip_fits(int nu, int nb, bool weights) {
 }
 template <typename T>
 int drift_strip_width(int nu, int want) {
-  if (sizeof(T) != 4 || want == DRIFT_WINDOW) return DRIFT_WINDOW;
-  const bool fit2 = strip_fits(nu, 2, false), fit1 = strip_fits(nu, 1, false);
+  if (want == DRIFT_WINDOW || (sizeof(T) == 8 && want == DRIFT_AUTO)) return DRIFT_WINDOW;
+  bool fit2, fit1;
+  if (sizeof(T) == 8) {
+    // 228 KB per SM, 1 KB of it reserved per block; the blocks' sums are static
+    const size_t n = strip64_smem(nu);
+    fit2 = 2 * (n + 16 * 32 * sizeof(double) + 1024) <= 233472;
+    fit1 = n + 32 * 32 * sizeof(double) <= 232448;
+  } else {
+    fit2 = strip_fits(nu, 2, false);
+    fit1 = strip_fits(nu, 1, false);
+  }
   if (want == DRIFT_STRIP2) return fit2 ? DRIFT_STRIP2 : DRIFT_WINDOW;
   if (want == DRIFT_STRIP1) return fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
   return fit2 ? DRIFT_STRIP2 : fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
 }
-int drift_strip_box_rows(int nu) { return strip_smem(nu, 1, 1, false).rows; }
+template <typename T>
+int drift_strip_box_rows(int nu) {
+  return sizeof(T) == 8 ? D64_ROWS : strip_smem(nu, 1, 1, false).rows;
+}
 
 template <int NW, int NB, int MINB, bool WEIGHTS>
 static cudaError_t drift_strip_go(const CUtensorMap *tmS, const float *C, float *f,
@@ -1520,6 +1652,30 @@ cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C,
     case DRIFT_STRIP1:
       return go(drift_strip_go<STRIP_WARPS, 1, 1, true>, drift_strip_go<STRIP_WARPS, 1, 1, false>,
                 1);
+    default:
+      return cudaErrorInvalidValue;
+  }
+}
+
+cudaError_t launch_drift_strip64(const CUtensorMap *tmS, int kind, const double *C, double *f,
+                                 const int32_t *idx, const double *fx, const double *fy,
+                                 const int64_t *ch_start, const int32_t *ch_len,
+                                 const double *ch_val, int64_t ndrift, const MomentTables &mt,
+                                 double *partial, unsigned int *err, uint32_t spins,
+                                 const Geometry &g, cudaStream_t st) {
+  const size_t smem = strip64_smem(g.nu);
+  auto go = [&](auto kern, int nw) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return chain_launch(kern, dim3(strip_blocks(g.nr), g.nb), dim3(32 * nw), smem, st, *tmS, C, f,
+                        idx, fx, fy, ch_start, ch_len, ch_val, ndrift, mt, partial, err, spins, g);
+  };
+  switch (kind) {
+    case DRIFT_STRIP2:
+      return go(drift_strip64_kernel<16, 2>, 16);
+    case DRIFT_STRIP1:
+      return go(drift_strip64_kernel<32, 1>, 32);
     default:
       return cudaErrorInvalidValue;
   }
@@ -1884,6 +2040,7 @@ cudaError_t launch_nonfinite(const T *f, size_t n, unsigned int *flag,
 
 #define VLS_INST(T)                                                            \
   template int drift_strip_width<T>(int, int);                                  \
+  template int drift_strip_box_rows<T>(int);                                    \
   template cudaError_t launch_drift_tma<T>(                                     \
       const CUtensorMap *, const T *, T *, const int32_t *, const T *, const T *, \
       const uint2 *, const int16_t *, const int64_t *, const int32_t *, const T *, \
