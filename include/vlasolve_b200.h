@@ -121,8 +121,8 @@ int vls_create(const vls_grid_desc *grid, const vls_solver_desc *solver,
                        where a line fits them, else shared-memory segments;
                        VLS_PREFILTER_SEGMENT: segments for every line.
      drift             VLS_DRIFT_AUTO: FP32 storage stages whole coefficient
-                       strips (two strip buffers per block where they fit,
-                       else one), FP64 storage and strips too tall for one
+                       strips (two strip buffers per SM where they fit, else
+                       one), FP64 storage and strips too tall for one
                        block take staged windows; VLS_DRIFT_WINDOW /
                        _STRIP2 / _STRIP1 ask for one of those (a strip that
                        does not fit falls back to windows).

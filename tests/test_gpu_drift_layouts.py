@@ -83,3 +83,51 @@ def test_fp64_strips_in_batches_are_bit_identical(drift):
     a.step(4)
     b.step(4)
     np.testing.assert_array_equal(a.f, b.f)
+
+
+@pytest.mark.parametrize("drift", ["strip2", "strip1"])
+@pytest.mark.parametrize("nr,nu", [(65, 33), (130, 97), (34, 112), (720, 47)])
+def test_short_fp32_strips_take_the_general_gather(nr, nu, drift):
+    """FP32 strips of fewer than 15 trips run in blocks of one strip, whose cells
+    take the general gather: the same bits as the windowed drift's."""
+    from vlasolve_b200 import VlasovSolver21Spline
+    cfg = _cfg(nr, nu, kernelBufferSize=2)
+    f = {}
+    for k in ("window", drift):
+        s = VlasovSolver21Spline(cfg, precision="fp32", layout={"drift": k})
+        assert s.layout()["drift"] == k
+        s.step(1)
+        s.sync()
+        f[k] = s.f
+    np.testing.assert_array_equal(f[drift], f["window"])
+
+
+@pytest.mark.parametrize("nr,nu", [(33, 33), (34, 112), (34, 113), (65, 97), (97, 129)])
+@pytest.mark.parametrize("drift", ["strip2", "strip1"])
+def test_strips_at_the_edge_of_the_block_form_match_oracle(nr, nu, drift):
+    from vlasolve_b200 import VlasovSolver21Spline
+    cfg = _cfg(nr, nu, kernelBufferSize=8)
+    a = VlasovSolver21Spline(cfg, precision="fp32", layout={"drift": drift})
+    b = VlasovSolver21Spline(cfg, precision="fp32",
+                             layout={"drift": drift, "slices_per_batch": 2, "streams": 2})
+    o = Oracle(cfg)
+    for _ in range(3):
+        for s in (a, b, o):
+            s.step(1)
+        _close(a, o, "fp32")
+    np.testing.assert_array_equal(a.f, b.f)
+
+
+@pytest.mark.parametrize("drift", ["strip2", "strip1"])
+def test_fp32_strip_blocks_wait_timeout_reports_and_falls_back(drift):
+    from vlasolve_b200 import VlasovSolver21Spline, _lib
+    cfg = _cfg(65, 33)
+    s = VlasovSolver21Spline(cfg, precision="fp32",
+                             layout={"drift": drift, "drift_wait_spins": -1})
+    o = Oracle(cfg)
+    s.step(1)
+    o.step(1)
+    with pytest.raises(_lib.VlsError) as e:
+        s.sync()
+    assert e.value.code == _lib.VLS_ECUDA and "drift" in str(e.value)
+    _close(s, o, "fp32")

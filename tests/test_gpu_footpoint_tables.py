@@ -115,10 +115,12 @@ def test_chains_and_far_cells_match_oracle(shape, precision, drift):
 
 
 @pytest.mark.parametrize("drift", ["strip2", "strip1"])
-def test_refilled_strip_buffers_match_oracle(drift):
+@pytest.mark.parametrize("nu", [33, 131])
+def test_refilled_strip_buffers_match_oracle(nu, drift):
     """More strips than twice the buffers of 148 SMs, so that every block
-    refills its buffers, with all three kinds of trips."""
-    cfg = _cfg(96, (32, 200), 0.05, kernelBufferSize=4)
+    refills its buffers (131 v_r vertices; shorter strips have a block each),
+    with all three kinds of trips."""
+    cfg = _cfg(96, (nu - 1, 200), 0.05, kernelBufferSize=4)
     t, _, _ = _tables_of(cfg)
     assert t["regular"].shape[0] * t["regular"].shape[1] > 2 * 2 * 148
     assert t["regular"].any() and t["empty"].any() and t["others"].any()

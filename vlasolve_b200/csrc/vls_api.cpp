@@ -97,6 +97,7 @@ struct vls_handle {
   CUtensorMap tmC[8];
   CUtensorMap tmS[8];  // and strips (drift_kind a strip kind)
   int drift_kind = DRIFT_WINDOW;
+  bool drift_blocks = false;  // strips in blocks, not by persistent ones
   uint32_t drift_spins = MBAR_SPIN_LIMIT;  // polls of each bounded wait of the drift
   vls_layout_desc layout{};                // what vls_get_layout reports
   // opt-in per-kernel event timing
@@ -326,8 +327,8 @@ static int footpoints_changed(vls_handle *h) {
   h->fp_gen++;
   const Coords &c = h->co;
   h->far_base_h.assign((size_t)c.nj + 1, 0);
-  if (h->esize == 8 && h->drift_kind != DRIFT_WINDOW) {
-    h->foot_ok = true;  // FP64 strips test every cell
+  if (h->drift_kind != DRIFT_WINDOW && h->drift_blocks) {
+    h->foot_ok = true;  // strips in blocks test every cell
     return VLS_OK;
   }
   if (h->drift_kind == DRIFT_WINDOW) {
@@ -557,10 +558,8 @@ static bool make_tensor_map(vls_handle *h) {
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return false;
     if (h->drift_kind != DRIFT_WINDOW) {
-      const cuuint32_t sbox[3] = {48,
-                                  (cuuint32_t)(es == 4 ? drift_strip_box_rows<float>(h->co.nu)
-                                                       : drift_strip_box_rows<double>(h->co.nu)),
-                                  1};
+      const cuuint32_t sbox[3] = {
+          48, (cuuint32_t)drift_strip_box_rows(h->co.nu, h->drift_blocks), 1};
       if (enc(&h->tmS[s],
               es == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
               base, dims, strides, sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -790,6 +789,8 @@ extern "C" int vls_create_layout(const vls_grid_desc *grid, const vls_solver_des
   // drift kernel: whole-strip staging where it fits (see vls_layout_desc)
   h->drift_kind = h->esize == 4 ? drift_strip_width<float>(c.nu, lay.drift)
                                 : drift_strip_width<double>(c.nu, lay.drift);
+  h->drift_blocks = h->esize == 4 ? drift_strip_in_blocks<float>(c.nr, c.nu)
+                                  : drift_strip_in_blocks<double>(c.nr, c.nu);
   h->drift_spins = lay.drift_wait_spins == 0  ? MBAR_SPIN_LIMIT
                    : lay.drift_wait_spins < 0 ? 0u
                                               : (uint32_t)lay.drift_wait_spins;
@@ -1228,13 +1229,12 @@ static int drift_once(vls_handle *h, bool kick, const void *f_in = nullptr,
     CK(h, timed(
               h, VLS_K_DRIFT,
               [&] {
-                if constexpr (sizeof(T) == 8) {
-                  if (h->drift_kind != DRIFT_WINDOW)
-                    return launch_drift_strip64(
-                        &h->tmS[sl], h->drift_kind, C, fout, h->idx, (const T *)h->fx,
-                        (const T *)h->fy, h->ch_start, h->ch_len, (const T *)h->ch_val, h->ndrift,
-                        moment_tables(h), h->partial, h->flag + 1, h->drift_spins, g, bs);
-                } else {
+                if (h->drift_kind != DRIFT_WINDOW && h->drift_blocks)
+                  return launch_drift_strip_blocks<T>(
+                      &h->tmS[sl], h->drift_kind, C, fout, h->idx, (const T *)h->fx,
+                      (const T *)h->fy, h->fp2, h->ch_start, h->ch_len, (const T *)h->ch_val,
+                      h->ndrift, moment_tables(h), h->partial, h->flag + 1, h->drift_spins, g, bs);
+                if constexpr (sizeof(T) == 4) {
                   if (h->drift_kind != DRIFT_WINDOW)
                     return launch_drift_strip(&h->tmS[sl], h->drift_kind, C, fout, h->fp2,
                                               h->trip_kinds, moment_tables(h), h->partial,

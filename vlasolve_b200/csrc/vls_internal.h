@@ -123,22 +123,27 @@ cudaError_t launch_window_rows(const int32_t *idx, const uint2 *fp2, int16_t *ro
 // columns x drift_strip_box_rows x 1 slice).  drift_strip_width returns the
 // strip kind (DRIFT_STRIP2 / DRIFT_STRIP1) the grid takes, or DRIFT_WINDOW
 // when none fits; want != DRIFT_AUTO requests one kind (FP64 takes strips on
-// request only, by a kernel of its own that reads the chains' fronts itself)
+// request only)
 template <typename T>
 int drift_strip_width(int nu, int want);
+// strips in blocks (drift_strip_block_kernel: FP64, and FP32 grids of short
+// strips) or by persistent blocks; the former read the chains' fronts and
+// their far taps themselves.  Rows of a box of tmS for either
 template <typename T>
-int drift_strip_box_rows(int nu);
+bool drift_strip_in_blocks(int nr, int nu);
+int drift_strip_box_rows(int nu, bool blocks);
 cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C, float *f,
                                const uint2 *fp2, const uint8_t *trip_kinds,
                                const MomentTables &mt, double *partial, unsigned int *err,
                                uint32_t spins, const Geometry &g, cudaStream_t st);
-cudaError_t launch_drift_strip64(const CUtensorMap *tmS, int kind, const double *C, double *f,
-                                 const int32_t *idx, const double *fx, const double *fy,
-                                 const int64_t *ch_start, const int32_t *ch_len,
-                                 const double *ch_val, int64_t ndrift, const MomentTables &mt,
-                                 double *partial, unsigned int *err, uint32_t spins,
-                                 const Geometry &g, cudaStream_t st);
-// what the FP32 strip drift knows of its footpoints (see vls_kernels.cu), from the
+template <typename T>
+cudaError_t launch_drift_strip_blocks(const CUtensorMap *tmS, int kind, const T *C, T *f,
+                                      const int32_t *idx, const T *fx, const T *fy,
+                                      const uint2 *fp2, const int64_t *ch_start,
+                                      const int32_t *ch_len, const T *ch_val, int64_t ndrift,
+                                      const MomentTables &mt, double *partial, unsigned int *err,
+                                      uint32_t spins, const Geometry &g, cudaStream_t st);
+// what the persistent strip drift knows of its footpoints (see vls_kernels.cu), from the
 // packed tables of all slices: the kind of each trip (bytes of that table,
 // and the kernel that fills it), and the cells of each slice whose taps leave
 // their strip (their number per slice, or with a list and its base per slice
@@ -150,9 +155,9 @@ cudaError_t launch_far_cells(const uint2 *fp2, const uint32_t *base, uint32_t *c
                              uint32_t *list, int nr, int nu, int nj, cudaStream_t st);
 // the chains (their ring, cell within the slice, tail footpoint; chain_lo:
 // first chain of each slice) and, for the strip drift, the far-tap cells
-// (far_base: first of each slice; nullptr for the windowed drift and FP64).
-// launch_edge advances every chain of the launch's slices and, for the strip
-// drift, writes the edge cells' values into f (edge_kernel)
+// (far_base: first of each slice; nullptr for every other drift).
+// launch_edge advances every chain of the launch's slices and, for the
+// persistent strip drift, writes the edge cells' values into f (edge_kernel)
 struct EdgeTables {
   const int64_t *ch_start;
   const int32_t *ch_len;

@@ -1465,31 +1465,35 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
   }
 }
 
-// FP64 strips, for handles that ask for them (VLS_DRIFT_STRIP2 / _STRIP1; the
-// windowed drift is the faster one and FP64's default: 513 x 513 x 128
-// Hernquist STRIP1 0.358 ms against 0.301, 257 x 253 x 128 STRIP2 0.100
-// against 0.095).  Block: 32 output columns x every row of one J slice; the
-// whole strip is staged in boxes of D64_ROWS rows, lanes walk the rows of a
-// column in turn, footpoints two rows ahead; cells whose taps leave the strip,
-// chain fronts and, after a wait that ran out, every cell are read in global
-// memory.
-constexpr int D64_ROWS = 64, D64_AHEAD = 2;
-template <int NW, int MINB>
+// Strips in blocks: 32 output columns x every row of one J slice per block,
+// the whole strip staged in boxes of DSB_ROWS rows; lanes walk the rows of
+// a column in turn, footpoints two rows ahead; a warp vote per two rows sends
+// the rare cells (taps outside the strip, chain fronts and, after a wait that
+// ran out, every cell) to global memory.
+//
+// For FP64 handles that ask for strips (the windowed drift is the faster one
+// and FP64's default: 513 x 513 x 128 Hernquist STRIP1 0.366 ms against 0.300,
+// 257 x 253 x 128 STRIP2 0.100 against 0.094), and for FP32 grids of short
+// strips (drift_strip_in_blocks).  What bounds it: 116 instructions per cell
+// in FP32, footpoint loads in FP64.
+constexpr int DSB_ROWS = 64, DSB_AHEAD = 2;
+template <typename T, int NW, int MINB>
 __global__ void __launch_bounds__(32 * NW, MINB)
-    drift_strip64_kernel(const __grid_constant__ CUtensorMap tmS, const double *C,
-                         double *__restrict__ f, const int32_t *__restrict__ idx,
-                         const double *__restrict__ fx, const double *__restrict__ fy,
-                         const int64_t *__restrict__ ch_start,
-                         const int32_t *__restrict__ ch_len, const double *ch_val,
-                         int64_t ndrift, MomentTables mt, double *__restrict__ partial,
-                         unsigned int *err, uint32_t spins, Geometry g) {
-  constexpr int WC = DS_WC, PF = D64_AHEAD;
+    drift_strip_block_kernel(const __grid_constant__ CUtensorMap tmS, const T *C,
+                             T *__restrict__ f, const int32_t *__restrict__ idx,
+                             const T *__restrict__ fx, const T *__restrict__ fy,
+                             const uint2 *__restrict__ fp2,
+                             const int64_t *__restrict__ ch_start,
+                             const int32_t *__restrict__ ch_len, const T *ch_val,
+                             int64_t ndrift, MomentTables mt, double *__restrict__ partial,
+                             unsigned int *err, uint32_t spins, Geometry g) {
+  constexpr int WC = DS_WC, PF = DSB_AHEAD;
   static_assert(NW * PF + 1 <= FOOT_PAD_ROWS, "the loads ahead reach past the padding rows");
-  constexpr uint32_t BYTES = D64_ROWS * WC * sizeof(double);
+  constexpr uint32_t BYTES = DSB_ROWS * WC * sizeof(T);
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ double red[NW][32];
-  const int rows = g.nu + 3, nch = (rows + D64_ROWS - 1) / D64_ROWS;
-  double *win = reinterpret_cast<double *>(smem_raw);
+  const int rows = g.nu + 3, nch = (rows + DSB_ROWS - 1) / DSB_ROWS;
+  T *win = reinterpret_cast<T *>(smem_raw);
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem_raw + (size_t)nch * BYTES);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int r0 = blockIdx.x * 32, r = r0 + lane, x0 = r0 - DS_XL;
@@ -1501,49 +1505,71 @@ __global__ void __launch_bounds__(32 * NW, MINB)
     mbar_fence_init();
     for (int c = 0; c < nch; ++c) {
       mbar_expect_tx(&bar[c], BYTES);
-      tma_load_3d(win + (size_t)c * D64_ROWS * WC, &tmS, x0, c * D64_ROWS, jl, &bar[c]);
+      tma_load_3d(win + (size_t)c * DSB_ROWS * WC, &tmS, x0, c * DSB_ROWS, jl, &bar[c]);
     }
   }
   __syncthreads();
-  const double *Cj = C + (size_t)jl * rows * g.pc;
-  bool staged = true;
-  for (int c = 0; c < nch && staged; ++c) staged = mbar_wait_bounded(&bar[c], 0u, spins);
-  if (!staged) atomicOr(err, 1u);
-  auto value = [&](const RawCell<double> &c) {
-    const Cell<double> cl = decode(c);
-    if (cl.kind == 0) {
-      const uint32_t wc = (uint32_t)(cl.rI - x0);
-      if (staged && wc < (uint32_t)(WC - 3))
-        return eval_pitch<WC>(win + cl.uI * WC + wc, cl.x, cl.y);
-      return eval2d<double>(Cj, g.pc, cl.rI, cl.x, cl.uI, cl.y);
-    }
-    if (cl.kind == 2) return ch_val[__ldg(ch_start + cl.ch) + ndrift % __ldg(ch_len + cl.ch)];
-    return 0.0;
+  const T *Cj = C + (size_t)jl * rows * g.pc;
+  auto weight = [&](int u) -> T {
+    if constexpr (sizeof(T) == 4)
+      return __ldg(mt.bu32 + u);
+    else
+      return __ldg(mt.bu + u);
   };
   // rows w, w + NW, ...; loads ahead run past the slice into the next one or
   // the tables' padding, and lanes past N_r read the next row's words
   const size_t sb = (size_t)j * g.nu * g.nr;
   const uint32_t step = (uint32_t)NW * (uint32_t)g.nr;
   uint32_t off = (uint32_t)w * (uint32_t)g.nr + (uint32_t)r;
-  RawCell<double> q[PF];
+  RawCell<T> q[PF];
 #pragma unroll
-  for (int k = 0; k < PF; ++k) q[k] = load_raw(idx + sb, fx + sb, fy + sb, nullptr, off + k * step);
+  for (int k = 0; k < PF; ++k) q[k] = load_raw(idx, fx, fy, fp2, sb + off + k * step);
+  bool staged = true;
+  for (int c = 0; c < nch && staged; ++c) staged = mbar_wait_bounded(&bar[c], 0u, spins);
+  if (!staged) atomicOr(err, 1u);
+  const uint32_t wcap = staged ? (uint32_t)(WC - 3) : 0u;
+  // the in-strip gather, run for every lane with the tap offset zeroed where
+  // it does not apply (rare: the value comes from slow instead)
+  auto fast = [&](const RawCell<T> &c, bool ok, bool &rare) {
+    const Cell<T> cl = decode(c);
+    const uint32_t wc = (uint32_t)(cl.rI - x0);
+    const bool in = ok && cl.kind == 0 && wc < wcap;
+    rare = ok && !in;
+    return eval_pitch<WC>(win + (in ? cl.uI * WC + (int)wc : 0), cl.x, cl.y);
+  };
+  auto slow = [&](const RawCell<T> &c) {
+    const Cell<T> cl = decode(c);
+    if (cl.kind == 0) return eval2d<T>(Cj, g.pc, cl.rI, cl.x, cl.uI, cl.y);
+    if (cl.kind == 2) return ch_val[__ldg(ch_start + cl.ch) + ndrift % __ldg(ch_len + cl.ch)];
+    return T(0);
+  };
   double acc = 0.0;
   for (int u = w; u < g.nu; u += NW * PF) {
-    double part = 0.0;
+    T v[PF];
+    RawCell<T> c[PF];
+    bool rare[PF], any = false;
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
-      const RawCell<double> c = q[k];
-      if (u + NW * k < g.nu)
-        q[k] = load_raw(idx + sb, fx + sb, fy + sb, nullptr, off + PF * step);
+      c[k] = q[k];
+      if (u + NW * k < g.nu) q[k] = load_raw(idx, fx, fy, fp2, sb + off + (PF + k) * step);
+      v[k] = fast(c[k], col_ok && u + NW * k < g.nu, rare[k]);
+      any |= rare[k];
+    }
+    if (__any_sync(0xffffffffu, any)) {
+#pragma unroll
+      for (int k = 0; k < PF; ++k)
+        if (rare[k]) v[k] = slow(c[k]);
+    }
+    T part = T(0);
+#pragma unroll
+    for (int k = 0; k < PF; ++k) {
       if (u + NW * k < g.nu && col_ok) {
-        const double v = value(c);
-        f[sb + off] = v;
-        part += __ldg(mt.bu + u + NW * k) * v;
+        f[sb + off] = v[k];
+        part += weight(u + NW * k) * v[k];
       }
       off += step;
     }
-    acc += part;
+    acc += (double)part;
   }
   // N_r = 32 k + 1: the last block also takes the last column, one row per
   // thread (its strip covers columns r0 - 8 .. r0 + 39)
@@ -1552,9 +1578,12 @@ __global__ void __launch_bounds__(32 * NW, MINB)
   if (extra)
     for (int u = tid; u < g.nu; u += 32 * NW) {
       const size_t cell = sb + (size_t)u * g.nr + r0 + 32;
-      const double v = value(load_raw(idx, fx, fy, nullptr, cell));
+      const RawCell<T> c = load_raw(idx, fx, fy, fp2, cell);
+      bool rare;
+      T v = fast(c, true, rare);
+      if (rare) v = slow(c);
       f[cell] = v;
-      acc2 += __ldg(mt.bu + u) * v;
+      acc2 += (double)(weight(u) * v);
     }
   // every box must have landed before the block's shared memory is released
   if (tid == 0)
@@ -1582,13 +1611,14 @@ __global__ void __launch_bounds__(32 * NW, MINB)
 }
 
 // Strip layouts (the DRIFT_* kinds).  FP32: DRIFT_STRIP2, two strip buffers
-// per block; DRIFT_STRIP1, one (strips too tall for two).  FP64: DRIFT_STRIP2,
-// two blocks of one strip per SM; DRIFT_STRIP1, one.  DRIFT_WINDOW: none, the
+// per persistent block; DRIFT_STRIP1, one (strips too tall for two).  Strips
+// in blocks: DRIFT_STRIP2, two blocks per SM; DRIFT_STRIP1, one.  DRIFT_WINDOW: none, the
 // windowed kernel, which FP64 takes unless a strip is asked for.  `want` !=
 // DRIFT_AUTO asks for one kind, returned only if it fits (else DRIFT_WINDOW).
-static size_t strip64_smem(int nu) {
-  const int nch = (nu + 3 + D64_ROWS - 1) / D64_ROWS;
-  return (size_t)nch * (D64_ROWS * DS_WC * sizeof(double) + sizeof(uint64_t));
+template <typename T>
+static size_t strip_block_smem(int nu) {
+  const int nch = (nu + 3 + DSB_ROWS - 1) / DSB_ROWS;
+  return (size_t)nch * (DSB_ROWS * DS_WC * sizeof(T) + sizeof(uint64_t));
 }
 static bool strip_fits(int nu, int nb, bool weights) {
   // 227 KB of shared memory per block with the barriers; strips of 576 and
@@ -1602,7 +1632,7 @@ int drift_strip_width(int nu, int want) {
   bool fit2, fit1;
   if (sizeof(T) == 8) {
     // 228 KB per SM, 1 KB of it reserved per block; the blocks' sums are static
-    const size_t n = strip64_smem(nu);
+    const size_t n = strip_block_smem<T>(nu);
     fit2 = 2 * (n + 16 * 32 * sizeof(double) + 1024) <= 233472;
     fit1 = n + 32 * 32 * sizeof(double) <= 232448;
   } else {
@@ -1613,9 +1643,22 @@ int drift_strip_width(int nu, int want) {
   if (want == DRIFT_STRIP1) return fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
   return fit2 ? DRIFT_STRIP2 : fit1 ? DRIFT_STRIP1 : DRIFT_WINDOW;
 }
+// Strips of fewer than 15 trips (N_u <= 112) leave most of the persistent
+// block's consumer warps without one, and each task costs its producer some
+// 3 us whatever its length (four or eight strip buffers instead of two change
+// nothing).  Drift in us, FP32 Hernquist, 128 slices, blocks / persistent:
+// 720 x 33 34.5 / 58.2, 395 x 33 22.9 / 37.4, 720 x 65 49.8 / 63.8, 257 x 97
+// 28.9 / 29.1, 720 x 105 65.1 / 70.0; 257 x 113 32.1 / 30.2, 129 x 129 24.3 /
+// 23.4, 257 x 257 56.4 / 45.4.  Blocks need no pass for the far cells either
+// (step of 257 x 97 x 128 59.5 us against 61.4).  Slices of one strip stay
+// with the persistent blocks (33 x 97 x 128 15.4 / 12.6).  The rule takes the
+// whole grid's sizes, not a batch's: results do not depend on the batching.
 template <typename T>
-int drift_strip_box_rows(int nu) {
-  return sizeof(T) == 8 ? D64_ROWS : strip_smem(nu, 1, 1, false).rows;
+bool drift_strip_in_blocks(int nr, int nu) {
+  return sizeof(T) == 8 || (strip_trips(nu) < 15 && strip_blocks(nr) > 1);
+}
+int drift_strip_box_rows(int nu, bool blocks) {
+  return blocks ? DSB_ROWS : strip_smem(nu, 1, 1, false).rows;
 }
 
 template <int NW, int NB, int MINB, bool WEIGHTS>
@@ -1657,25 +1700,27 @@ cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C,
   }
 }
 
-cudaError_t launch_drift_strip64(const CUtensorMap *tmS, int kind, const double *C, double *f,
-                                 const int32_t *idx, const double *fx, const double *fy,
-                                 const int64_t *ch_start, const int32_t *ch_len,
-                                 const double *ch_val, int64_t ndrift, const MomentTables &mt,
-                                 double *partial, unsigned int *err, uint32_t spins,
-                                 const Geometry &g, cudaStream_t st) {
-  const size_t smem = strip64_smem(g.nu);
+template <typename T>
+cudaError_t launch_drift_strip_blocks(const CUtensorMap *tmS, int kind, const T *C, T *f,
+                                      const int32_t *idx, const T *fx, const T *fy,
+                                      const uint2 *fp2, const int64_t *ch_start,
+                                      const int32_t *ch_len, const T *ch_val, int64_t ndrift,
+                                      const MomentTables &mt, double *partial, unsigned int *err,
+                                      uint32_t spins, const Geometry &g, cudaStream_t st) {
+  const size_t smem = strip_block_smem<T>(g.nu);
   auto go = [&](auto kern, int nw) {
     const cudaError_t e =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     return chain_launch(kern, dim3(strip_blocks(g.nr), g.nb), dim3(32 * nw), smem, st, *tmS, C, f,
-                        idx, fx, fy, ch_start, ch_len, ch_val, ndrift, mt, partial, err, spins, g);
+                        idx, fx, fy, fp2, ch_start, ch_len, ch_val, ndrift, mt, partial, err,
+                        spins, g);
   };
   switch (kind) {
     case DRIFT_STRIP2:
-      return go(drift_strip64_kernel<16, 2>, 16);
+      return go(drift_strip_block_kernel<T, 16, 2>, 16);
     case DRIFT_STRIP1:
-      return go(drift_strip64_kernel<32, 1>, 32);
+      return go(drift_strip_block_kernel<T, 32, 1>, 32);
     default:
       return cudaErrorInvalidValue;
   }
@@ -2040,7 +2085,12 @@ cudaError_t launch_nonfinite(const T *f, size_t n, unsigned int *flag,
 
 #define VLS_INST(T)                                                            \
   template int drift_strip_width<T>(int, int);                                  \
-  template int drift_strip_box_rows<T>(int);                                    \
+  template bool drift_strip_in_blocks<T>(int, int);                             \
+  template cudaError_t launch_drift_strip_blocks<T>(                            \
+      const CUtensorMap *, int, const T *, T *, const int32_t *, const T *, const T *, \
+      const uint2 *, const int64_t *, const int32_t *, const T *, int64_t,       \
+      const MomentTables &, double *, unsigned int *, uint32_t, const Geometry &, \
+      cudaStream_t);                                                            \
   template cudaError_t launch_drift_tma<T>(                                     \
       const CUtensorMap *, const T *, T *, const int32_t *, const T *, const T *, \
       const uint2 *, const int16_t *, const int64_t *, const int32_t *, const T *, \
