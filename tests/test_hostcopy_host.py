@@ -2,7 +2,7 @@
 does nothing before it must: queued copies run when their event or stream is
 waited for, so a chunk that is filled again or emptied too early gives wrong
 bytes.  Element by element, around the chunks' borders, from several threads,
-and where no memory can be page-locked."""
+where no memory can be page-locked, and with a single thread."""
 
 import os
 import shutil
@@ -119,13 +119,20 @@ int main(int argc, char **argv) {
     for (unsigned k = 0; k < 5; ++k)
       t.emplace_back([=] { for (unsigned i = 0; i < 3; ++i) roundtrip(M + k * C + 8 * i, 8 * k, 31 * k + i); });
     for (std::thread &x : t) x.join();
-  } else {
+  } else if (std::atoi(argv[1]) == 2) {
     // no page-locked memory at all, then one block (half a pair), then enough
     for (int left : {0, 1, 1 << 20}) {
       allocs_left = left;
       roundtrip(M + 3 * C + 8, 8, (unsigned)left);
       if (cudaGetLastError() != cudaSuccess) ++bad;
     }
+  }
+  if (std::atoi(argv[1]) == 3) {
+    // one thread: no chunks
+    staged = 0;
+    allocs_left = 0;
+    roundtrip(M + 3 * C + 8, 8, 5);
+    if (staged || allocs_left != 0) ++bad;
   }
   if (!locked.empty()) ++bad;  // the last object gave the chunks back
   std::printf("%d\n", bad);
@@ -147,8 +154,12 @@ def exe(tmp_path_factory):
     return str(d / "t")
 
 
-@pytest.mark.parametrize("case", ["borders", "threads", "no_locked_memory"])
+CASES = ["borders", "threads", "no_locked_memory", "one_thread"]
+
+
+@pytest.mark.parametrize("case", CASES)
 def test_copies(exe, case):
-    n = ["borders", "threads", "no_locked_memory"].index(case)
-    r = subprocess.run([exe, str(n)], capture_output=True, text=True, timeout=300)
+    env = dict(os.environ, OMP_NUM_THREADS="1" if case == "one_thread" else "4")
+    r = subprocess.run([exe, str(CASES.index(case))], capture_output=True, text=True, timeout=300,
+                       env=env)
     assert r.returncode == 0, r.stdout + r.stderr
