@@ -1933,7 +1933,7 @@ cudaError_t launch_scan(const double *partial, const MomentTables &mt,
 
 // ------------------------------------------------------------------ stats
 // integrate() of Ek, S, L1, L2 (quadrature21.hxx:56-85, integrand21.hxx:82-145)
-// Block: one J slice, ST_U rows of u cells; a thread takes one r cell and
+// Block: one J slice, stats_rows rows of u cells; a thread takes one r cell and
 // walks down the rows, so that the radius' terms (J^2 / rm^2, a division) are
 // formed once and each f row pair is loaded once.  Every term enters its sum
 // compensated; block partials in double-double, 4 quantities x (hi, lo).
@@ -1941,19 +1941,26 @@ cudaError_t launch_scan(const double *partial, const MomentTables &mt,
 // compensated sums): 513 x 513 x 256 FP32 0.555 -> 0.359 ms (the whole call,
 // its final sums and copies included, 1.11 -> 0.39 ms) against 8-row blocks
 // with the division, five loads and renormalised sums per cell.
+//
+// 16 rows a block, fewer where those blocks leave SMs idle (two per SM wanted:
+// the whole call on 2048 x 33 x 8 FP32 61 us, 110 with 16 rows always).
 constexpr int ST_THREADS = 256;
-constexpr int ST_U = 16;
+static int stats_rows(int nu, int nj) {
+  int rows = 16;
+  while (rows > 2 && (int64_t)((nu - 1 + rows - 1) / rows) * nj < 2 * 148) rows /= 2;
+  return rows;
+}
 
 template <typename T>
 __global__ void __launch_bounds__(ST_THREADS)
     stats_kernel(const T *f, const double *__restrict__ R,
                  const double *__restrict__ U, const double *__restrict__ J,
                  const double *__restrict__ dR, const double *__restrict__ dU,
-                 const double *__restrict__ Ct1, double *__restrict__ part,
+                 const double *__restrict__ Ct1, double *__restrict__ part, int rows,
                  Geometry g) {
   chain_begin();
   const int j = blockIdx.y;
-  const int u0 = blockIdx.x * ST_U, u1 = min(u0 + ST_U, g.nu - 1);
+  const int u0 = blockIdx.x * rows, u1 = min(u0 + rows, g.nu - 1);
   dd acc[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
   const double Jj = __ldg(J + j), ct = __ldg(Ct1 + j);
   for (int r = threadIdx.x; r < g.nr - 1 && u0 < u1; r += ST_THREADS) {
@@ -2017,16 +2024,20 @@ __global__ void __launch_bounds__(ST_THREADS)
   }
 }
 
-size_t stats_blocks(int nu, int nj) { return (size_t)((nu - 1 + ST_U - 1) / ST_U) * nj; }
+size_t stats_blocks(int nu, int nj) {
+  const int rows = stats_rows(nu, nj);
+  return (size_t)((nu - 1 + rows - 1) / rows) * nj;
+}
 
 template <typename T>
 cudaError_t launch_stats(const T *f, const double *R, const double *U,
                          const double *J, const double *dR, const double *dU,
                          const double *Ct1, double *part, double *out4,
                          const Geometry &g, cudaStream_t st) {
-  dim3 grid((g.nu - 1 + ST_U - 1) / ST_U, g.nj);
+  const int rows = stats_rows(g.nu, g.nj);
+  dim3 grid((g.nu - 1 + rows - 1) / rows, g.nj);
   const cudaError_t e = chain_launch(stats_kernel<T>, grid, dim3(ST_THREADS), 0, st, f, R, U, J,
-                                     dR, dU, Ct1, part, g);
+                                     dR, dU, Ct1, part, rows, g);
   if (e != cudaSuccess) return e;
   return chain_launch(stats_sum_kernel, dim3(4), dim3(ST_THREADS), 0, st, part,
                       (int)stats_blocks(g.nu, g.nj), out4);
