@@ -125,3 +125,23 @@ def test_refilled_strip_buffers_match_oracle(nu, drift):
     assert t["regular"].shape[0] * t["regular"].shape[1] > 2 * 2 * 148
     assert t["regular"].any() and t["empty"].any() and t["others"].any()
     _compare(cfg, "fp32", drift)
+
+
+@pytest.mark.parametrize("nr", [33, 65, 160, 192, 257])
+def test_long_runs_of_strips_are_those_of_short_ones(nr):
+    """More than 12 strips for each of 148 blocks are taken in another order than
+    fewer; values and moments are those of batches of few slices, bit for bit."""
+    from vlasolve_b200 import VlasovSolver21Spline
+    ns = nr // 32 if nr % 32 == 1 else -(-nr // 32)
+    nj = -(-12 * 148 // ns) + 7
+    cfg = _cfg(nr - 1, (112, nj), 0.02, kernelBufferSize=3)
+    a = VlasovSolver21Spline(cfg, precision="fp32", layout={"drift": "strip2"})
+    b = VlasovSolver21Spline(cfg, precision="fp32",
+                             layout={"drift": "strip2", "slices_per_batch": 61})
+    for _ in range(2):
+        a.step(1)
+        b.step(1)
+        assert a.last_mass() == b.last_mass()
+        np.testing.assert_array_equal(a.f, b.f)
+    a.sync()
+    b.sync()

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <numeric>
 
 #include "vls_async.cuh"
 #include "vls_dd.cuh"
@@ -1221,7 +1222,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
                        float *f, const uint2 *__restrict__ fp2,
                        const uint8_t *__restrict__ trip_kinds, MomentTables mt,
                        double *__restrict__ partial, unsigned int *err, uint32_t spins,
-                       Geometry g) {
+                       uint32_t rot, Geometry g) {
   constexpr int WC = DS_WC;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ uint64_t full[NB], done[NB];
@@ -1247,14 +1248,19 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
   if constexpr (WEIGHTS)
     for (int u = tid; u < nt * DS_TRIP; u += 32 * (NW + 1)) wsm[u] = __ldg(mt.bu32 + u);
   __syncthreads();
-  const int nmine = (int)blockIdx.x < ntask ? (ntask - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  // this block's i-th task: one of the i-th gridDim.x tasks in turn
+  auto task_of = [&](int i) {
+    return i * (int)gridDim.x + (int)((blockIdx.x + (uint32_t)i * rot) % gridDim.x);
+  };
+  const int whole = ntask / (int)gridDim.x;
+  const int nmine = whole + (task_of(whole) < ntask ? 1 : 0);
 
   if (w == NW) {  // ------------------------------------------------ producer
     // a strip's boxes; then its trips' kinds (into registers, then into the
     // buffer), and its share of its slice's footpoint words into L2, where
     // the trips find them a strip or two later, in flight DS_AHEAD rows ahead
     auto issue = [&](int i) {
-      const int task = (int)blockIdx.x + i * (int)gridDim.x, b = i % NB;
+      const int task = task_of(i), b = i % NB;
       const int jl = task / ns, sx = task - jl * ns;
       if (lane == 0) {
         mbar_expect_tx(&full[b], (uint32_t)L.strip);
@@ -1273,14 +1279,14 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
     constexpr int KPL = 5;  // kinds per lane: strips of up to 1280 rows
     uint8_t kd[KPL];
     auto fetch = [&](int i) {
-      const int task = (int)blockIdx.x + i * (int)gridDim.x;
+      const int task = task_of(i);
       const int jl = task / ns, sx = task - jl * ns;
       const uint8_t *src = trip_kinds + ((size_t)(g.j0 + jl) * ns + sx) * nt;
 #pragma unroll
       for (int k = 0; k < KPL; ++k) kd[k] = lane + 32 * k < nt ? __ldg(src + lane + 32 * k) : 0;
     };
     auto words_to_l2 = [&](int i) {
-      const int task = (int)blockIdx.x + i * (int)gridDim.x;
+      const int task = task_of(i);
       const int jl = task / ns, sx = task - jl * ns;
       const uint64_t lo = (uint64_t)(g.j0 + jl) * g.nu * g.nr * 8u;
       const uint64_t n = (uint64_t)g.nu * g.nr * 8u, part = (n / (ns * 32u) + 31u) & ~15ull;
@@ -1320,7 +1326,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
         fence_proxy_async();
         issue(issued);
       }
-      const int task = (int)blockIdx.x + i * (int)gridDim.x;
+      const int task = task_of(i);
       const int jl = task / ns, sx = task - jl * ns, j = g.j0 + jl;
       const double *red = buf_red(b);
       double sum = 0.0, sumx = 0.0;
@@ -1361,7 +1367,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
     return fp2 + ((size_t)(g.j0 + jl) * g.nu + DS_TRIP * t) * nr +
            min(sx * 32 + lane, g.nr - 1);
   };
-  int task = (int)blockIdx.x;
+  int task = task_of(0);
   if (nmine > 0) {
     load_q(words(task, min(first_trip(task), nt - 1)));
   }
@@ -1369,7 +1375,7 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
     const int b = i % NB;
     const int jl = task / ns, sx = task - jl * ns, j = g.j0 + jl;
     const int x0 = sx * 32 - DS_XL;
-    const int tnext = (int)(task + (int)gridDim.x);
+    const int tnext = task_of(i + 1);
     const float *win = buf_win(b);
     const unsigned char *kinds = kinds0 + b * L.kinds;
     const bool ok = __all_sync(
@@ -1661,6 +1667,35 @@ int drift_strip_box_rows(int nu, bool blocks) {
   return blocks ? DSB_ROWS : strip_smem(nu, 1, 1, false).rows;
 }
 
+// A block's tasks are task b of the first `grid` ones, task (b + rot) % grid of
+// the next, and so on: its strip moves by (grid + rot) % ns each time.  148
+// blocks and 32 strips without rotation give every block 8 of the 32 strips,
+// whose cost differs by a factor of six, so blocks drift apart in a long run:
+// the drift of 1025 x 1025 x 512 PLDF took 5.28 us a slice (4.70 with 128
+// slices), of 513 x 513 x 2048 1.24 (256: 1.06).  With steps coprime to ns and
+// between 0.2 and 0.45 of it from either side 4.55 and 0.89, 513 x 513 x 256
+// Hernquist 0.263 -> 0.248 ms; a step of one strip is worse than none (1025 x
+// 1025 x 64 0.377 against 0.303), and so is one of half of them (0.326).
+// Rotations from 3 on are the better ones in shorter runs (513 x 513 x 256
+// 0.248 with 3, 0.253 with 1; 1025 x 1025 x 64 0.300 and 0.313), from 1 on where
+// a larger one would go round the blocks more than once (1025 x 1025 x 512 4.92
+// and 4.55).  Runs of fewer than 12 tasks a block keep the plain order: there
+// the last tasks decide (257 x 352 x 128 0.060, rotated 0.064; 257 x 257 x 128
+// 0.049, 0.047).
+static int strip_rotation(int ntask, int grid, int ns) {
+  if (ntask < 12 * grid) return 0;
+  auto far = [&](int rot) {
+    const int step = (grid + rot) % ns, near = std::min(step, ns - step);
+    return std::gcd(step, ns) == 1 && 5 * near >= ns && 20 * near <= 9 * ns;
+  };
+  const int first = ntask < 60 * grid ? 3 : 1;
+  for (int rot = 0; rot < first + ns; rot += rot ? 1 : first)
+    if (far(rot)) return rot;
+  for (int rot = 0; rot < ns; ++rot)  // 2 and 6 strips
+    if (std::gcd(grid + rot, ns) == 1) return rot;
+  return 0;
+}
+
 template <int NW, int NB, int MINB, bool WEIGHTS>
 static cudaError_t drift_strip_go(const CUtensorMap *tmS, const float *C, float *f,
                                   const uint2 *fp2, const uint8_t *trip_kinds,
@@ -1675,9 +1710,10 @@ static cudaError_t drift_strip_go(const CUtensorMap *tmS, const float *C, float 
   if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
   if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
     return e;
-  const int ntask = strip_blocks(g.nr) * g.nb;
-  return chain_launch(kern, dim3(std::min(ntask, nsm * MINB)), dim3(32 * (NW + 1)), smem, st, *tmS,
-                      C, f, fp2, trip_kinds, mt, partial, err, spins, g);
+  const int ns = strip_blocks(g.nr), ntask = ns * g.nb, grid = std::min(ntask, nsm * MINB);
+  const int rot = strip_rotation(ntask, grid, ns);
+  return chain_launch(kern, dim3(grid), dim3(32 * (NW + 1)), smem, st, *tmS, C, f, fp2, trip_kinds,
+                      mt, partial, err, spins, (uint32_t)rot, g);
 }
 
 cudaError_t launch_drift_strip(const CUtensorMap *tmS, int kind, const float *C, float *f,
