@@ -181,7 +181,10 @@ int vls_get_f(vls_handle *h, double *host, size_t n);
    (vlasovSolver21_spline.hxx:69-72, :88-100) and disp_driftOut
    (vlasovSolver21.hxx:94, :140-143); each array has N_r*N_u*N_J entries.
    Any pointer may be NULL.  vls_set_footpoints replaces the tables (driftR is
-   only used for the kernel-radius test). */
+   only used for the kernel-radius test) and what the drift derives from them;
+   it waits for the device and may allocate.  VLS_EINVAL leaves the tables as
+   they were; after any other error the handle refuses to step or to run a
+   backward pass (VLS_ESTATE) until they are set again. */
 int vls_get_footpoints(const vls_handle *h, int32_t *rI, double *rF,
                        int32_t *uI, double *uF, uint8_t *out, double *driftR);
 int vls_set_footpoints(vls_handle *h, const int32_t *rI, const double *rF,

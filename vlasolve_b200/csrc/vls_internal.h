@@ -17,7 +17,7 @@
 //                                     (second word = chain id)
 //   the footpoint tables end with FOOT_PAD_ROWS zeroed rows of N_r cells and
 //   32 more zeroed cells past the last slice, so that the strip drift
-//   prefetches the next rows of a slice without clamping the row index
+//   loads the next rows of a slice without clamping the row index
 //   chains: ch_start/int64, ch_len/int32 per chain, ch_val/T per element
 //           (ring buffer; logical front at (ndrift mod len)), tail footpoint
 //   partial [N_J][N_r] double       per-slice radial moment partial sums
@@ -30,12 +30,15 @@
 
 namespace vls {
 
-// a bounded mbarrier wait gives up after ~2^20 polls (tens of milliseconds
-// at most)
+// a bounded mbarrier wait gives up after 2^20 polls: tens of milliseconds, and
+// some 0.2 s for the waits that sleep 100 ns between polls (mbar_wait_idle; a
+// block whose copies never land takes a few of them, one after another)
 constexpr uint32_t MBAR_SPIN_LIMIT = 1u << 20;
 
-// readable rows past the end of the footpoint tables (the strip drift reads
-// at most 16 warps x 2 rows ahead; 32 cells more cover the lanes past N_r)
+// readable rows past the end of the footpoint tables: strips in blocks read up
+// to 32 warps x 2 rows ahead (32 cells more cover the lanes past N_r), the
+// persistent strips the rest of a trip, and their prefetch into L2 ends less
+// than N_u / 32 rows and 32 bytes past the last slice
 constexpr int FOOT_PAD_ROWS = 66;
 
 // Thomas tables of one direction of the natural-BC cubic B-spline solve
@@ -99,7 +102,10 @@ constexpr int DRIFT_AUTO = 0, DRIFT_WINDOW = 1, DRIFT_STRIP2 = 2, DRIFT_STRIP1 =
 // the windowed drift's staged windows, columns x rows of coefficients (the
 // box of its tensor map).  FP64 drift of 513 x 513 x 128 / 201 x 201 x 200:
 // 48 x 48 0.305 / 0.0946 ms, 48 x 40 0.308 / 0.0958, 48 x 56 0.311 / 0.0942,
-// 64 x 32 0.315 / 0.0977, 64 x 40 0.313 / 0.0980, 64 x 48 0.410 / 0.110
+// 64 x 32 0.315 / 0.0977, 64 x 40 0.313 / 0.0980, 64 x 48 0.410 / 0.110.
+// FP32 lines too long for a strip, 513 x 1537 x 64 / 257 x 2048 x 64: 48 x 48
+// 0.478 / 0.450, 64 x 40 0.483 / 0.460, 64 x 48 0.485 / 0.459, 48 x 40 0.486 /
+// 0.458
 constexpr int DW_COLS = 48, DW_ROWS = 48;
 // footpoints: FP64 handles use idx/fx/fy, FP32 handles the packed fp2 table.
 // Drift with the coefficient windows staged by TMA (tmC: 3D map of C, box

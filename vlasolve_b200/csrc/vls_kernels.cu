@@ -6,10 +6,13 @@
 //             u, kick gather at U+shift(r), second solve along u of the kicked
 //             values -> G (u-direction coefficients of the kicked f)
 //   prer      per (J slice, rows of G): solve along r -> C (2D coefficients)
+//   edge      per delayed-kernel chain: spline value at the chain tail; for the
+//             persistent strip drift also the chain fronts' and the far cells'
+//             values, into f
 //   drift     per cell: 4x4 gather of C at the host-tabulated footpoint, or the
-//             delayed-kernel ring-buffer front, or 0; radial moment partials
-//             of the result (the next step's moment) in the epilogue
-//   tails     per delayed-kernel chain: spline value at the chain tail
+//             delayed-kernel ring-buffer front (persistent strips: what edge
+//             left in f), or 0; radial moment partials of the result (the next
+//             step's moment) in the epilogue
 //
 // The 2D prefilter of the reference (r-solves, then u-solves on every column,
 // localSpline.hxx:1238-1258) is applied here as u-solves then r-solves; the
@@ -950,10 +953,12 @@ __host__ __device__ inline int strip_blocks(int nr) {
 __host__ __device__ inline int strip_trips(int nu) { return (nu + DS_TRIP - 1) / DS_TRIP; }
 constexpr int DS_WC = 48, DS_XL = (DS_WC - 32) / 2;  // columns staged, and left of the strip
 // consumer warps of a block (one producer warp besides) and footpoint rows in
-// flight per warp: drift of 513 x 513 x 256 Hernquist / 257 x 257 x 128
-// Plummer with 31 warps and two rows (64 registers) 0.295 / 0.061 ms, 23 and
-// four (80 registers) 0.270 / 0.053, 19 and four (96) 0.261 / 0.049, 17 and
-// four 0.277 / 0.051, 13 and four 0.309 / 0.052, 19 and eight 0.282 / 0.051
+// flight per warp.  Drift of 513 x 513 x 256 Hernquist / 257 x 257 x 128
+// Plummer / 395 x 307 x 77 UDF / 1025 x 1025 x 64 PLDF in us, four rows: 17
+// warps 261 / 51.4 / 55.7 / 313, 19 (96 registers) 249 / 48.4 / 53.9 / 300, 21
+// 260 / 51.5 / 53.8 / 318, 23 (80) 252 / 51.7 / 53.6 / 298.  In an earlier form
+// (plain order of the tasks) 31 warps and two rows took 295 / 61, 13 and four
+// 309 / 52, 19 and eight 282 / 51.
 constexpr int STRIP_WARPS = 19;
 constexpr int DS_AHEAD = 4;
 
@@ -1206,11 +1211,11 @@ __host__ __device__ inline StripSmem strip_smem(int nu, int nw, int nb, bool wei
 //
 // What bounds it: about 60 instructions per cell in regular trips and 110 in
 // the others at some 60 % of the issue slots, and a quarter of the time waits
-// for a strip.  A block per strip with 16 x 2 warps per SM, every cell with
-// its 16 taps and the rare cells gathered in place, took 0.309 ms on the 513 x
-// 513 x 256 Hernquist case, 0.372 on 1025 x 1025 x 64 PLDF and 0.057 on 257 x
-// 257 x 128 Plummer (116 instructions per cell); this form 0.261, 0.306 and
-// 0.049, and edge_kernel 0.012, 0.018 and 0.000 more than the tails alone.
+// for a strip.  drift_strip_block_kernel (a block per strip, every cell with
+// its 16 taps and the rare cells gathered in place; 116 instructions per cell)
+// took 0.311 ms on the 513 x 513 x 256 Hernquist case, 0.373 on 1025 x 1025 x
+// 64 PLDF and 0.057 on 257 x 257 x 128 Plummer; this form 0.249, 0.300 and
+// 0.048, and edge_kernel 0.012, 0.018 and 0.001 more than the tails alone.
 //
 // Waits are bounded.  A consumer whose wait for a strip ran out (`spins`
 // polls) gathers that strip's cells from global memory; the producer waits
@@ -1270,11 +1275,12 @@ __global__ void __launch_bounds__(32 * (NW + 1), MINB)
       }
       __syncwarp();
     };
-    // into L2 only for strips of up to 352 rows: then the words, coefficients
-    // and values of the strips in flight on the whole chip stay well inside
-    // it (drift 257 x 257 x 128 0.0486 ms with, 0.0523 without; 395 x 307 x
-    // 77 0.0537 and 0.0552; 513 x 513 x 256 0.261 and 0.257; 1025 x 1025 x 64
-    // 0.316 and 0.305)
+    // into L2 only for strips of up to 352 rows, a line found by measuring.
+    // Drift in us with / without: 257 x 257 x 128 48.5 / 51.6, 395 x 307 x 77
+    // 54.0 / 55.2, 257 x 352 x 128 60.2 / 62.9, 257 x 384 x 128 65.6 / 67.2;
+    // 513 x 441 x 128 119.5 / 118.4, 513 x 513 x 256 260 / 249, 1025 x 1025 x
+    // 64 317 / 300.  Few strips in flight do not move it: 513 x 513 x 32 56.2 /
+    // 55.3, 1025 x 1025 x 8 59.5 / 58.2.
     const bool l2_words = g.nu <= 352;
     constexpr int KPL = 5;  // kinds per lane: strips of up to 1280 rows
     uint8_t kd[KPL];
